@@ -14,6 +14,8 @@
 
 #include <vector>
 
+#include "oa_ell.cuh"
+
 namespace oa {
 
 template <class T>
@@ -36,8 +38,8 @@ struct AmgLevel {
   int *pt_rp = nullptr, *pt_rows = nullptr, *pt_src = nullptr;
   T* ptv = nullptr;  // P^T values in coarse-row order
   int nnz_p = 0;
-  // lanes per row of the row-parallel kernels (1, 8 or 32, from the average
-  // row length): A, P, P^T, and the T / coarse term lists
+  // lanes per row of the row-parallel kernels (from the average row length):
+  // A, P, P^T, and the T / coarse term lists
   int lpr_a = 1, lpr_p = 1, lpr_pt = 1, lpr_t = 1, lpr_c = 1;
   // T = A P values and term lists (A entry, P entry); the next level's values
   // from term lists (P entry, T entry)
@@ -49,21 +51,25 @@ struct AmgLevel {
   // (residual), t (pre-smoothed iterate)
   T *x = nullptr, *b = nullptr, *r = nullptr, *t = nullptr;
   // Chebyshev smoother (small levels): preconditioned residual, two direction
-  // buffers; the power-iteration estimate of the spectral radius of Dinv A
-  // (lmax[1]) and its FP64 work arrays (matrix and Dinv copies, two vectors,
-  // block partials)
+  // buffers; the power-iteration state (est[0] = 1 / |v|, est[1] = the bound of
+  // the spectral radius of Dinv A), its FP64 vectors and block partials, and
+  // the step coefficients formed from the bound (coef[0] = 1 / theta, then
+  // c1, c2 of steps 1 .. MAX_CHEB - 1)
   bool cheb = false;
   T *cr = nullptr, *cd0 = nullptr, *cd1 = nullptr;
-  double* lmax = nullptr;
-  double *pw_a = nullptr, *pw_dinv = nullptr, *pw_v = nullptr, *pw_w = nullptr, *pw_part = nullptr;
+  double *est = nullptr, *coef = nullptr;
+  double *pw_v = nullptr, *pw_w = nullptr, *pw_part = nullptr;
+  unsigned* pw_ticket = nullptr;
   bool own_A = false;
+  // level 0: the caller's matrix in fixed-width storage (null: CSR)
+  EllGraph ell;
+  const T* ell_val = nullptr;
 };
 
 template <class T>
 struct Amg {
   std::vector<AmgLevel<T>> L;
-  double* dense_inv = nullptr;    // coarsest level inverse (FP64, n x n)
-  double* h_dense = nullptr;      // pinned staging
+  double* dense_inv = nullptr;    // coarsest level: [A | I], then its inverse in the right half (FP64, n x 2n)
   int coarse_n = 0;
   bool smoothed = true;           // smoothed (true) or piecewise-constant prolongation
   double omega = 0.8;             // Jacobi damping of the smoother
@@ -79,7 +85,12 @@ struct Amg {
   int cheb_degree = 3;
   int cheb_rows = 50000;
   double cheb_ratio = 30.0;
-  long long cheb_launches = 0;    // extra launches per V-cycle of the Chebyshev levels
+  // the cycle from level `tail` down is one dense operator [n][n] (row-major),
+  // formed by the numeric phase in dense_work
+  int tail = 0;
+  double* dense_op = nullptr;
+  double* dense_work = nullptr;
+  int dense_operator(cudaStream_t st);
   bool ready = false;
 
   // structure from the fine graph (host arrays); device pointers of the fine
@@ -93,6 +104,12 @@ struct Amg {
   // before set-up they shape it, after it they take effect with the next
   // numeric phase (degree) and apply (launch count)
   int set_smoothing(int degree, double prolongation_damping);
+  // fixed-width storage of the current finest matrix (null: its CSR arrays are used)
+  void set_finest(const EllGraph& g, const T* val) {
+    if (L.empty()) return;
+    L[0].ell = g;
+    L[0].ell_val = val;
+  }
   void release();
   ~Amg() { release(); }
 };

@@ -42,6 +42,16 @@ __global__ void k_correct_clip(int n, double* phi, const double* x, double lo) {
   phi[i] = v;
 }
 
+// The momentum solution in FP64, and (U given) the velocity correction
+template <class T>
+__global__ void k_momentum_apply(int n, const T* __restrict__ x, double* __restrict__ x64, double* U) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double v = double(x[i]);
+  x64[i] = v;
+  if (U) U[i] += 1.0 * v;
+}
+
 __global__ void k_axpy(int n, double* y, const double* x, double a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] += a * x[i];
@@ -213,8 +223,7 @@ template <class T>
 int momentum_control(oa_flow* h, const T* b, const T* r, int iters) {
   Flow& f = h->f;
   const int nn = f.mesh->nn;
-  if (int s = device_comp_sumsq3<T>(nn, b, h->scal + 2, f.red, f.stream)) return s;
-  if (int s = device_comp_sumsq3<T>(nn, r, h->scal + 5, f.red, f.stream)) return s;
+  if (int s = device_comp_sumsq3<T>(nn, b, r, h->scal + 2, f.red, f.stream)) return s;
   OA_CUDA(cudaMemcpyAsync(h->hscal + 2, h->scal + 2, 6 * sizeof(double), cudaMemcpyDeviceToHost, f.stream));
   OA_CUDA(cudaStreamSynchronize(f.stream));
   oa_control_data& cd = f.cd_mom;
@@ -241,7 +250,7 @@ int solve_momentum(oa_flow* h, double rtol, int maxit, int* iters, double* res, 
     if (int s = h->mom32.solve<float>(static_cast<const float*>(f.b.A_mom), static_cast<const float*>(f.b.b_mom), x,
                                       rtol, maxit, &it, res, 10))
       return s;
-    k_to_double<float><<<(3 * m.nn + 255) / 256, 256, 0, f.stream>>>(3 * (size_t)m.nn, x, f.b.x_mom);
+    k_momentum_apply<float><<<(3 * m.nn + 255) / 256, 256, 0, f.stream>>>(3 * m.nn, x, f.b.x_mom, apply ? f.U : nullptr);
     count_launches(1);
     if (int s = momentum_control<float>(h, static_cast<const float*>(f.b.b_mom), h->mom32.residual(), it)) return s;
   } else {
@@ -250,12 +259,11 @@ int solve_momentum(oa_flow* h, double rtol, int maxit, int* iters, double* res, 
     if (int s = h->mom64.solve<double>(static_cast<const double*>(f.b.A_mom),
                                        static_cast<const double*>(f.b.b_mom), x, rtol, maxit, &it, res, 10))
       return s;
-    OA_CUDA(cudaMemcpyAsync(f.b.x_mom, x, sizeof(double) * 3 * m.nn, cudaMemcpyDeviceToDevice, f.stream));
+    k_momentum_apply<double><<<(3 * m.nn + 255) / 256, 256, 0, f.stream>>>(3 * m.nn, x, f.b.x_mom, apply ? f.U : nullptr);
+    count_launches(1);
     if (int s = momentum_control<double>(h, static_cast<const double*>(f.b.b_mom), h->mom64.residual(), it)) return s;
   }
   if (iters) *iters = it;
-  if (apply) k_axpy<<<(3 * m.nn + 255) / 256, 256, 0, f.stream>>>(3 * m.nn, f.U, f.b.x_mom, 1.0);
-  count_launches(1);
   OA_CUDA(cudaGetLastError());
   return OA_OK;
 }
@@ -283,6 +291,7 @@ ScalarGraph pc_graph(const DeviceMesh& m) {
   g.h_rp = m.h_row_ptr.data();
   g.h_cols = m.h_cols.data();
   g.h_diag = m.h_diag.data();
+  g.ell = m.ell;
   return g;
 }
 
@@ -392,22 +401,18 @@ int build_iteration_graph(oa_flow* h) {
   // assembly with the rhs norm
   if (int s = gb.seg(g, d, -1, [&]() -> int {
         if (mx) {
-          k_to_double<float><<<(n3 + 255) / 256, 256, 0, f.stream>>>((size_t)n3, h->mom32.solution(), f.b.x_mom);
-          count_launches(1);
-          if (int s2 = device_comp_sumsq3<float>(m.nn, static_cast<const float*>(f.b.b_mom), G.dsum, f.red, f.stream))
+          k_momentum_apply<float><<<(n3 + 255) / 256, 256, 0, f.stream>>>(n3, h->mom32.solution(), f.b.x_mom, f.U);
+          if (int s2 = device_comp_sumsq3<float>(m.nn, static_cast<const float*>(f.b.b_mom), h->mom32.residual(),
+                                                 G.dsum, f.red, f.stream))
             return s2;
-          if (int s2 = device_comp_sumsq3<float>(m.nn, h->mom32.residual(), G.dsum + 3, f.red, f.stream)) return s2;
           OA_CUDA(cudaMemcpyAsync(G.mom_host, h->mom32.scalars(), sizeof(KScal), cudaMemcpyDeviceToHost, f.stream));
         } else {
-          OA_CUDA(cudaMemcpyAsync(f.b.x_mom, h->mom64.solution(), sizeof(double) * n3, cudaMemcpyDeviceToDevice,
-                                  f.stream));
-          if (int s2 = device_comp_sumsq3<double>(m.nn, static_cast<const double*>(f.b.b_mom), G.dsum, f.red,
-                                                  f.stream))
+          k_momentum_apply<double><<<(n3 + 255) / 256, 256, 0, f.stream>>>(n3, h->mom64.solution(), f.b.x_mom, f.U);
+          if (int s2 = device_comp_sumsq3<double>(m.nn, static_cast<const double*>(f.b.b_mom), h->mom64.residual(),
+                                                  G.dsum, f.red, f.stream))
             return s2;
-          if (int s2 = device_comp_sumsq3<double>(m.nn, h->mom64.residual(), G.dsum + 3, f.red, f.stream)) return s2;
           OA_CUDA(cudaMemcpyAsync(G.mom_host, h->mom64.scalars(), sizeof(KScal), cudaMemcpyDeviceToHost, f.stream));
         }
-        k_axpy<<<(n3 + 255) / 256, 256, 0, f.stream>>>(n3, f.U, f.b.x_mom, 1.0);
         count_launches(1);
         if (int s2 = mark(2)) return s2;
         if (int s2 = launch_update_mdot(f, true)) return s2;
@@ -718,7 +723,8 @@ int oa_mesh_create(const double* coords, int nn, const int* conn, int ne, int to
     oa_mesh_destroy(M);
     return fail(OA_ERR_CUDA, std::string("mesh upload: ") + cudaGetErrorString(ce));
   }
-  if ((st = launch_geometry(m, M->st))) {
+  if ((st = ell_graph(nn, m.h_row_ptr.data(), m.row_ptr, m.cols, &m.ell, M->st)) ||
+      (st = launch_geometry(m, M->st))) {
     oa_mesh_destroy(M);
     return st;
   }
@@ -731,7 +737,7 @@ void oa_mesh_destroy(oa_mesh* M) {
   DeviceMesh& m = M->m;
   void* ptrs[] = {m.x,       m.conn,      m.n2e,      m.n2e_ptr,  m.n2f,       m.n2f_ptr, m.face_elem, m.face_ord,
                   m.face_bnd, m.row_ptr, m.cols,     m.diag,     m.face_mask, m.vol,     m.wscv,      m.wall_node,
-                  m.scs_area, m.slot_mask, m.slot_mask64};
+                  m.scs_area, m.slot_mask, m.slot_mask64, const_cast<int*>(m.ell.cols)};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (M->st) cudaStreamDestroy(M->st);

@@ -162,6 +162,7 @@ int create_tet4_mesh(oa_mesh* M, const double* coords, int nn, const int* conn, 
   cudaError_t ce = cudaDeviceSynchronize();
   if (ce == cudaSuccess) ce = cudaGetLastError();
   if (ce != cudaSuccess) return fail(OA_ERR_CUDA, std::string("tet4 mesh upload: ") + cudaGetErrorString(ce));
+  if ((st = ell_graph(nn, m.h_row_ptr.data(), m.row_ptr, m.cols, &m.ell, M->st))) return st;
   // dual volumes
   double* scv = nullptr;
   int* err = nullptr;
@@ -519,6 +520,7 @@ int diff_solve(oa_diffusion* H, double rtol, int maxit, int* iters, double* res,
   g.h_rp = m.h_row_ptr.data();
   g.h_cols = m.h_cols.data();
   g.h_diag = m.h_diag.data();
+  g.ell = m.ell;
   return H->solver.solve(g, dmixed(H), H->s.amg != 0, H->s.use_graphs != 0, H->A, H->b, H->x, rtol, maxit, iters,
                          res, refinements, H->stream, "diffusion");
 }

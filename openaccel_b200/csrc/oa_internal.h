@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/openaccel_b200.h"
+#include "oa_ell.cuh"
 
 namespace oa {
 
@@ -60,6 +61,7 @@ struct DeviceMesh : MeshView {
   // hex8 elements relabelled into a consistently oriented block: the cube
   // rotation applied to each (empty when none was needed)
   std::vector<uint8_t> h_rot;
+  EllGraph ell;  // fixed-width storage of the stencil graph, where it has one
   // host copies needed for set-up and parity dumps
   std::vector<int> h_row_ptr, h_cols, h_diag;
   std::vector<int> h_conn, h_face_elem, h_face_ord, h_face_bnd;

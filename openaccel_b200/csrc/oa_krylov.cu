@@ -15,111 +15,107 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include <algorithm>
 #include <cmath>
+#include <vector>
 #include <type_traits>
 
 #include "oa_internal.h"
 #include "oa_krylov.h"
+#include "oa_ell.cuh"
 
 namespace oa {
 
 constexpr int KB = 256;        // threads per block for vector kernels
-constexpr int MAX_PARTIALS = 2048;
+// Blocks of the kernels that reduce (8 per SM; they loop over the rows), so
+// that the kernel which uses a sum can add the partials itself, in every block
+constexpr int MAX_PARTIALS = 8 * 148;
 
-template <class T>
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
 }
 
-// block-level fixed-order reduction of up to 3 values; thread 0 writes partials
+// Fixed-order two-stage reductions: a partial per block, and every block of
+// the kernel that needs the sum adds the partials in the same order. On a
+// 16^3 cavity this costs 0.1 to 0.2 us per kernel; a ticket with the last block
+// adding up cost 1.6 us, a kernel of one block for the sum 3 to 4.
 template <int NV>
-__device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* partials, int nblocks_stride) {
+__device__ __forceinline__ void block_partials(double (&v)[NV], double* partials) {
   __shared__ double sh[NV][KB / 32];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    double s = warp_sum<double>(v[k]);
+    const double s = warp_sum(v[k]);
     if (l == 0) sh[k][w] = s;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < NV) {
+    double s = 0.0;
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double s = 0.0;
-      for (int i = 0; i < KB / 32; ++i) s += sh[k][i];
-      partials[k * nblocks_stride + blockIdx.x] = s;
-    }
+    for (int i = 0; i < KB / 32; ++i) s += sh[threadIdx.x][i];
+    partials[threadIdx.x * MAX_PARTIALS + blockIdx.x] = s;
   }
 }
 
-// ordered final sum of the partials by one block
+// ordered sum of nb partials per value, in every thread
 template <int NV>
-__device__ __forceinline__ void final_reduce(const double* partials, int nb, double (&out)[NV]) {
-  __shared__ double sh[NV][KB];
+__device__ __forceinline__ void sum_partials(const double* __restrict__ partials, int nb, double (&out)[NV]) {
+  __shared__ double sh[NV][KB / 32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  double t[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) t[k] = 0.0;
+  for (int i = threadIdx.x; i < nb; i += KB)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) t[k] += __ldg(partials + k * MAX_PARTIALS + i);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const double s = warp_sum(t[k]);
+    if (l == 0) sh[k][w] = s;
+  }
+  __syncthreads();
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     double s = 0.0;
-    for (int i = threadIdx.x; i < nb; i += KB) s += partials[k * MAX_PARTIALS + i];
-    sh[k][threadIdx.x] = s;
-  }
-  __syncthreads();
-  for (int st = KB / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st)
 #pragma unroll
-      for (int k = 0; k < NV; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + st];
-    __syncthreads();
+    for (int i = 0; i < KB / 32; ++i) s += sh[k][i];
+    out[k] = s;
   }
-#pragma unroll
-  for (int k = 0; k < NV; ++k) out[k] = sh[k][0];
 }
 
-// y = A x for a BSR matrix with BxB row-major blocks; optional partial dots
-// (y.w1 and, for ND = 2, y.y).
-template <int B, class TM, class TV, int ND>
-__global__ void __launch_bounds__(KB) k_spmv(int nn, const int* __restrict__ rp, const int* __restrict__ cols,
-                                              const TM* __restrict__ A, const TV* __restrict__ x,
-                                              TV* __restrict__ y, const TV* __restrict__ w1,
-                                              const TV* __restrict__ w2, double* partials, const KScal* sc) {
-  if (sc && sc->done) return;
-  double v[ND > 0 ? ND : 1];
+static int reduce_grid(long long n) { return (int)std::min<long long>((n + KB - 1) / KB, MAX_PARTIALS); }
+
+// Product of row component m of block row [a, e) with x: U entries at a time
+// with every load in flight before the first use, summed in entry order.
+template <int B, class TM, class TV>
+__device__ __forceinline__ double row_product(const int* __restrict__ cols, const TM* __restrict__ A,
+                                              const TV* __restrict__ x, int a, int e, int m) {
+  constexpr int U = B == 1 ? 4 : (sizeof(TM) == 8 ? 2 : 4);
+  double s = 0.0;
+  for (int k = a; k < e; k += U) {
+    int j[U];
+    TM v[U][B];
 #pragma unroll
-  for (int k = 0; k < (ND > 0 ? ND : 1); ++k) v[k] = 0.0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nn * B; t += gridDim.x * blockDim.x) {
-    const int i = t / B, m = t - i * B;
-    double s = 0.0;
-    const int a = __ldg(rp + i), bnd = __ldg(rp + i + 1);
-    for (int k = a; k < bnd; ++k) {
-      const int j = __ldg(cols + k);
+    for (int u = 0; u < U; ++u) {
+      const int q = min(k + u, e - 1);
+      j[u] = __ldg(cols + q);
 #pragma unroll
-      for (int q = 0; q < B; ++q) s += double(A[(size_t)k * B * B + B * m + q]) * double(x[B * j + q]);
+      for (int c = 0; c < B; ++c) v[u][c] = __ldg(A + (size_t)q * B * B + B * m + c);
     }
-    const TV ys = TV(s);
-    y[t] = ys;
-    // second dot is y.y, taken from the register (never re-read through y)
-    if (ND > 0) v[0] += double(ys) * double(w1[t]);
-    if (ND > 1) v[1] += double(ys) * double(ys);
+    TV xv[U][B];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int c = 0; c < B; ++c) xv[u][c] = __ldg(x + (size_t)B * j[u] + c);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + u < e)
+#pragma unroll
+        for (int c = 0; c < B; ++c) s += double(v[u][c]) * double(xv[u][c]);
   }
-  if (ND > 0) block_reduce_store<ND>(reinterpret_cast<double(&)[ND]>(v), partials, MAX_PARTIALS);
-}
-
-// z = Minv v (point or 3x3 block Jacobi); the inverse is stored in the
-// precision of the Krylov vectors (FP32 in the mixed form's inner solves)
-template <int B, class TV>
-__global__ void k_prec(int nn, const TV* __restrict__ Minv, const TV* __restrict__ v, TV* __restrict__ z,
-                       const KScal* sc) {
-  if (sc->done) return;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nn * B) return;
-  if (B == 1) {
-    z[t] = TV(double(Minv[t]) * double(v[t]));
-  } else {
-    const int i = t / 3, m = t - 3 * i;
-    const TV* M = Minv + 9 * (size_t)i + 3 * m;
-    z[t] = TV(double(M[0]) * double(v[3 * i]) + double(M[1]) * double(v[3 * i + 1]) +
-              double(M[2]) * double(v[3 * i + 2]));
-  }
+  return s;
 }
 
 template <int B, class TM, class TP>
@@ -149,21 +145,19 @@ __global__ void k_build_minv(int nn, const int* __restrict__ rp, const int* __re
   }
 }
 
-// init: x = 0, r = rh = b, p = v = 0; partial ||b||^2
+// x = 0, r = b, and for BiCGStab rh = b (the directions start with the first
+// iteration, which reads none); partial ||b||^2
 template <class TV, class TB>
-__global__ void __launch_bounds__(KB) k_init(int n, const TB* __restrict__ b, TV* x, TV* r, TV* rh, TV* p, TV* v,
-                                              double* partials) {
+__global__ void __launch_bounds__(KB) k_init(int n, const TB* __restrict__ b, TV* x, TV* r, TV* rh, double* partials) {
   double s[1] = {0.0};
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const TV bv = TV(b[t]);
     x[t] = TV(0);
     r[t] = bv;
-    rh[t] = bv;
-    p[t] = TV(0);
-    v[t] = TV(0);
+    if (rh) rh[t] = bv;
     s[0] += double(bv) * double(bv);
   }
-  block_reduce_store<1>(s, partials, MAX_PARTIALS);
+  block_partials<1>(s, partials);
 }
 
 // rtol_dev / maxit_dev (when not null) replace rtol / maxit: the inner solves
@@ -171,7 +165,7 @@ __global__ void __launch_bounds__(KB) k_init(int n, const TB* __restrict__ b, TV
 __global__ void __launch_bounds__(KB) k_init_scalars(KScal* sc, const double* partials, int nb, double rtol,
                                                       int maxit, const double* rtol_dev, const int* maxit_dev) {
   double o[1];
-  final_reduce<1>(partials, nb, o);
+  sum_partials<1>(partials, nb, o);
   if (threadIdx.x == 0) {
     sc->rtol = rtol_dev ? *rtol_dev : rtol;
     sc->maxit = maxit_dev ? *maxit_dev : maxit;
@@ -181,140 +175,275 @@ __global__ void __launch_bounds__(KB) k_init_scalars(KScal* sc, const double* pa
     sc->d0 = o[0];  // rh.r for the first iteration equals ||b||^2
     sc->iters = 0;
     sc->status = 0;
+    sc->seg_rel = 0.0;
     sc->done = (sc->bnorm == 0.0 || !(sc->bnorm < INFINITY)) ? 1 : 0;
     if (!(sc->bnorm < INFINITY)) sc->status = 2;
   }
 }
 
-// p = r + beta (p - omega v), beta = (rho1/rho)(alpha/omega), rho1 = sc->d0
-template <class TV>
-__global__ void k_p_update(int n, TV* p, const TV* r, const TV* v, const KScal* sc) {
-  if (sc->done) return;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const double beta = (sc->d0 / sc->rho) * (sc->alpha / sc->omega);
-  p[t] = TV(double(r[t]) + beta * (double(p[t]) - sc->omega * double(v[t])));
-}
-
-// alpha = rho1 / (rh.v)
-__global__ void __launch_bounds__(KB) k_alpha(KScal* sc, const double* partials, int nb) {
-  if (sc->done) return;
-  double o[1];
-  final_reduce<1>(partials, nb, o);
-  if (threadIdx.x == 0) {
-    if (o[0] == 0.0 || !(fabs(o[0]) < INFINITY)) {
-      sc->done = 1;
-      sc->status = 1;
-      return;
+// z = Minv v of row i (point or 3x3 block Jacobi); the inverse is stored in
+// the precision of the Krylov vectors (FP32 in the mixed form's inner solves)
+template <int B, class TV>
+__device__ __forceinline__ void jacobi_row(const TV* __restrict__ Minv, int i, const TV (&v)[B], TV* z) {
+  if (B == 1) {
+    z[i] = TV(double(__ldg(Minv + i)) * double(v[0]));
+  } else {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const TV* M = Minv + 9 * (size_t)i + 3 * m;
+      z[3 * (size_t)i + m] = TV(double(__ldg(M)) * double(v[0]) + double(__ldg(M + 1)) * double(v[1 % B]) +
+                                double(__ldg(M + 2)) * double(v[2 % B]));
     }
-    sc->alpha = sc->d0 / o[0];
   }
 }
 
-// s = r - alpha v (stored in r)
-template <class TV>
-__global__ void k_s_update(int n, TV* r, const TV* v, const KScal* sc) {
+// p = r + beta (p - omega v), beta = (rho1/rho)(alpha/omega), rho1 = sc->d0
+// (p = r in the first iteration), and with Jacobi ph = Minv p; one thread per
+// row
+template <int B, class TV>
+__global__ void __launch_bounds__(KB) k_p_update(int nn, TV* p, const TV* __restrict__ r, const TV* __restrict__ v,
+                                                  const TV* __restrict__ Minv, TV* ph, const KScal* sc) {
   if (sc->done) return;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  r[t] = TV(double(r[t]) - sc->alpha * double(v[t]));
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nn) return;
+  const bool first = sc->iters == 0;
+  const double omega = sc->omega, beta = (sc->d0 / sc->rho) * (sc->alpha / omega);
+  TV q[B];
+#pragma unroll
+  for (int c = 0; c < B; ++c) {
+    const size_t t = (size_t)B * i + c;
+    q[c] = first ? r[t] : TV(double(r[t]) + beta * (double(p[t]) - omega * double(v[t])));
+    p[t] = q[c];
+  }
+  if (Minv) jacobi_row<B, TV>(Minv, i, q, ph);
 }
 
-// omega = (t.s)/(t.t)
-__global__ void __launch_bounds__(KB) k_omega(KScal* sc, const double* partials, int nb) {
+// alpha = rho1 / (rh.v) from the product's partials (a zero or non-finite rh.v
+// is a breakdown), s = r - alpha v (stored in r), and with Jacobi sh = Minv s
+template <int B, class TV>
+__global__ void __launch_bounds__(KB) k_s_update(int nn, TV* r, const TV* __restrict__ v,
+                                                  const TV* __restrict__ Minv, TV* sh,
+                                                  const double* __restrict__ partials, int nb, KScal* sc) {
+  if (sc->done) return;
+  double o[1];
+  sum_partials<1>(partials, nb, o);
+  const bool broken = o[0] == 0.0 || !(fabs(o[0]) < INFINITY);
+  const double alpha = broken ? 0.0 : sc->d0 / o[0];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (broken) {
+      sc->done = 1;
+      sc->status = 1;
+    } else {
+      sc->alpha = alpha;
+    }
+  }
+  if (broken) return;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
+    TV q[B];
+#pragma unroll
+    for (int c = 0; c < B; ++c) {
+      const size_t t = (size_t)B * i + c;
+      q[c] = TV(double(r[t]) - alpha * double(v[t]));
+      r[t] = q[c];
+    }
+    if (Minv) jacobi_row<B, TV>(Minv, i, q, sh);
+  }
+}
+
+// Row i of a scalar matrix times x
+template <class TM>
+struct ScalarMat {
+  const int *rp, *cols;  // CSR
+  const TM* A;
+  const int* ecols;      // fixed-width storage
+  const TM* eval;
+};
+template <int FORMAT, class TM, class TX>
+__device__ __forceinline__ double scalar_row(const ScalarMat<TM>& m, int i, const TX* __restrict__ x) {
+  if constexpr (FORMAT >= ELL)
+    return ell_row<FORMAT, TM>(m.ecols, m.eval, i, [&](int j) { return double(__ldg(x + j)); });
+  else
+    return row_product<1, TM, TX>(m.cols, m.A, x, __ldg(m.rp + i), __ldg(m.rp + i + 1), 0);
+}
+
+// a kernel template over the formats of a scalar matrix
+#define OA_FORMAT(format, call)        \
+  switch (format) {                    \
+    case ELL + 7: call(ELL + 7); break;                \
+    case ELL + 15: call(ELL + 15); break;              \
+    case ELL_STREAM + 7: call(ELL_STREAM + 7); break;  \
+    case ELL_STREAM + 15: call(ELL_STREAM + 15); break;\
+    default: call(1);                  \
+  }
+
+// y = A x for a BSR matrix with BxB row-major blocks.
+// STEP 1: partial w.y with w = rh; STEP 2: partials y.w and y.y with w = s.
+template <int B, class TM, class TV, int STEP, int FORMAT>
+__global__ void __launch_bounds__(KB, B == 1 ? 8 : 1) k_spmv(int nn, ScalarMat<TM> M, const TV* __restrict__ x, TV* __restrict__ y,
+                                              const TV* __restrict__ w, double* partials, const KScal* sc) {
+  if (sc->done) return;
+  double v[STEP];
+#pragma unroll
+  for (int k = 0; k < STEP; ++k) v[k] = 0.0;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nn * B; t += gridDim.x * blockDim.x) {
+    const double wt = double(w[t]);
+    double s;
+    if (B == 1) {
+      s = scalar_row<FORMAT, TM, TV>(M, t, x);
+    } else {
+      const int i = t / B, m = t - i * B;
+      s = row_product<B, TM, TV>(M.cols, M.A, x, __ldg(M.rp + i), __ldg(M.rp + i + 1), m);
+    }
+    const TV ys = TV(s);
+    y[t] = ys;
+    v[0] += double(ys) * wt;
+    if (STEP > 1) v[STEP - 1] += double(ys) * double(ys);
+  }
+  block_partials<STEP>(v, partials);
+}
+
+// End of a BiCGStab iteration: rho <- rho1; rho1 <- rh.r; convergence test
+// (per segment for batched systems)
+__device__ __forceinline__ void bicgstab_end(KScal* sc, double rr, double rhr, double segmax, int nseg) {
+  sc->seg_rel = segmax;
+  sc->rho = sc->d0;
+  sc->d0 = rhr;
+  sc->rnorm = sqrt(rr);
+  sc->iters += 1;
+  if (!(sc->rnorm < INFINITY)) {
+    sc->done = 1;
+    sc->status = 2;
+  } else if (sc->rnorm > 1e3 * sc->bnorm) {
+    sc->done = 1;  // diverging (seen with FP32 vectors on stiff systems)
+    sc->status = 3;
+  } else if ((nseg > 1 ? segmax <= sc->rtol : sc->rnorm <= sc->rtol * sc->bnorm) || sc->iters >= sc->maxit) {
+    sc->done = 1;
+  } else if (sc->omega == 0.0 || sc->d0 == 0.0) {
+    sc->done = 1;
+    sc->status = 1;
+  }
+}
+
+// End of a GCR iteration: residual norm and convergence test; an iteration that
+// leaves the residual where it was (truncated GCR can stagnate when the
+// preconditioned operator's symmetric part is not definite) ends the solve
+// with status 1, and the caller falls back to BiCGStab
+__device__ __forceinline__ void gcr_end(KScal* sc, double rr, double segmax, int nseg) {
+  sc->seg_rel = segmax;
+  const double prev = sc->rnorm;
+  sc->rnorm = sqrt(rr);
+  sc->iters += 1;
+  if (!(sc->rnorm < INFINITY)) {
+    sc->done = 1;
+    sc->status = 2;
+  } else if ((nseg > 1 ? segmax <= sc->rtol : sc->rnorm <= sc->rtol * sc->bnorm) || sc->iters >= sc->maxit) {
+    sc->done = 1;
+  } else if (sc->rnorm > 0.9999 * prev) {
+    sc->done = 1;
+    sc->status = 1;
+  }
+}
+
+// the partials of an iteration's last kernel close it
+template <bool GCR>
+__global__ void __launch_bounds__(KB) k_end_iter(KScal* sc, const double* partials, int nb) {
   if (sc->done) return;
   double o[2];
-  final_reduce<2>(partials, nb, o);
-  if (threadIdx.x == 0) sc->omega = o[1] > 0.0 ? o[0] / o[1] : 0.0;
+  if (GCR) {
+    double p[1];
+    sum_partials<1>(partials, nb, p);
+    o[0] = p[0];
+  } else {
+    sum_partials<2>(partials, nb, o);
+  }
+  if (threadIdx.x) return;
+  if (GCR) gcr_end(sc, o[0], 0.0, 0);
+  else bicgstab_end(sc, o[0], o[1], 0.0, 0);
 }
 
-// x += alpha ph + omega sh; r = s - omega t; partials r.r, rh.r
+// omega = (t.s)/(t.t) from the product's partials, x += alpha ph + omega sh,
+// r = s - omega t; partials r.r, rh.r
 template <class TV>
-__global__ void __launch_bounds__(KB) k_x_update(int n, TV* x, TV* r, const TV* ph, const TV* sh, const TV* t,
-                                                  const TV* rh, double* partials, const KScal* sc) {
+__global__ void __launch_bounds__(KB) k_x_update(int n, TV* x, TV* r, const TV* __restrict__ ph,
+                                                  const TV* __restrict__ sh, const TV* __restrict__ t,
+                                                  const TV* __restrict__ rh, const double* __restrict__ in, int nb,
+                                                  double* partials, KScal* sc) {
   if (sc->done) return;
+  double o[2];
+  sum_partials<2>(in, nb, o);
+  const double alpha = sc->alpha, omega = o[1] > 0.0 ? o[0] / o[1] : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc->omega = omega;
   double v[2] = {0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    x[i] = TV(double(x[i]) + sc->alpha * double(ph[i]) + sc->omega * double(sh[i]));
-    const TV rn = TV(double(r[i]) - sc->omega * double(t[i]));
+    x[i] = TV(double(x[i]) + alpha * double(ph[i]) + omega * double(sh[i]));
+    const TV rn = TV(double(r[i]) - omega * double(t[i]));
     r[i] = rn;
     v[0] += double(rn) * double(rn);
     v[1] += double(rh[i]) * double(rn);
   }
-  block_reduce_store<2>(v, partials, MAX_PARTIALS);
+  block_partials<2>(v, partials);
 }
 
-// Largest sqrt(r2[s] / b2[s]) over the segments (0 where b2 = 0), by the
-// whole block; 0 when nseg <= 1.
-__device__ __forceinline__ double block_seg_max(const double* r2, const double* b2, int nseg) {
-  __shared__ double sm[KB];
-  double m = 0.0;
-  if (nseg > 1)
-    for (int q = threadIdx.x; q < nseg; q += KB) {
-      const double b = b2[q];
-      if (b > 0.0) m = fmax(m, sqrt(r2[q] / b));
-    }
-  sm[threadIdx.x] = m;
-  __syncthreads();
-  for (int st = KB / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + st]);
-    __syncthreads();
-  }
-  return sm[0];
-}
-
-// per-segment sums of squares, one block per segment, fixed-order tree
-template <class T>
-__global__ void __launch_bounds__(KB) k_seg_sumsq(const int* __restrict__ ptr, const int* __restrict__ rows,
-                                                   const T* __restrict__ v, double* out, const int* done) {
-  if (done && *done) return;
-  __shared__ double sm[KB];
-  const int sg = blockIdx.x;
+// Segments of a batch: one block per chunk of a segment's rows sums squares,
+// and the last block adds each segment's chunks in order into out[] and takes
+// the largest sqrt(out[s] / b2[s]) (0 where b2 = 0). END 0: sums only (b2 may be
+// null); 1, 2: the convergence test that closes a BiCGStab / GCR iteration;
+// 3: the ratio into *ratio.
+template <class T, int END>
+__global__ void __launch_bounds__(KB) k_segments(Segments sg, const T* __restrict__ v, double* out, const double* b2,
+                                                  KScal* sc, double* ratio, const double* __restrict__ partials,
+                                                  int nb) {
+  if (END == 1 || END == 2)
+    if (sc->done) return;
+  __shared__ double sh[KB / 32];
+  __shared__ bool last;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int q1 = sg.chunk[blockIdx.x + 1];
   double a = 0.0;
-  for (int q = ptr[sg] + threadIdx.x; q < ptr[sg + 1]; q += KB) {
-    const double x = double(v[rows[q]]);
+  for (int q = sg.chunk[blockIdx.x] + threadIdx.x; q < q1; q += KB) {
+    const double x = double(v[__ldg(sg.rows + q)]);
     a += x * x;
   }
-  sm[threadIdx.x] = a;
+  a = warp_sum(a);
+  if (l == 0) sh[w] = a;
   __syncthreads();
-  for (int st = KB / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sm[threadIdx.x] += sm[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[sg] = sm[0];
-}
-
-__global__ void __launch_bounds__(KB) k_seg_max_ratio(const double* r2, const double* b2, int nseg, double* out) {
-  const double m = block_seg_max(r2, b2, nseg);
-  if (threadIdx.x == 0) *out = m;
-}
-
-// rho <- rho1; rho1 <- rh.r; convergence test (per segment for batched systems)
-__global__ void __launch_bounds__(KB) k_end_iter(KScal* sc, const double* partials, int nb, const double* seg_r2,
-                                                  const double* seg_b2, int nseg) {
-  if (sc->done) return;
-  double o[2];
-  final_reduce<2>(partials, nb, o);
-  const double segmax = block_seg_max(seg_r2, seg_b2, nseg);
   if (threadIdx.x == 0) {
-    sc->seg_rel = segmax;
-    const bool conv = nseg > 1 ? segmax <= sc->rtol : false;
-    sc->rho = sc->d0;
-    sc->d0 = o[1];
-    sc->rnorm = sqrt(o[0]);
-    sc->iters += 1;
-    if (!(sc->rnorm < INFINITY)) {
-      sc->done = 1;
-      sc->status = 2;
-    } else if (sc->rnorm > 1e3 * sc->bnorm) {
-      sc->done = 1;  // diverging (seen with FP32 vectors on stiff systems)
-      sc->status = 3;
-    } else if ((nseg > 1 ? conv : sc->rnorm <= sc->rtol * sc->bnorm) || sc->iters >= sc->maxit) {
-      sc->done = 1;
-    } else if (sc->omega == 0.0 || sc->d0 == 0.0) {
-      sc->done = 1;
-      sc->status = 1;
+    double s = 0.0;
+    for (int i = 0; i < KB / 32; ++i) s += sh[i];
+    sg.part[blockIdx.x] = s;
+    __threadfence();
+    last = atomicInc(sg.ticket, gridDim.x - 1) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double m = 0.0;
+  for (int s = threadIdx.x; s < sg.nseg; s += KB) {
+    double t = 0.0;
+    for (int c = sg.chunk_ptr[s]; c < sg.chunk_ptr[s + 1]; ++c) t += __ldcg(sg.part + c);
+    out[s] = t;
+    if (END) {
+      const double b = b2[s];
+      if (b > 0.0) m = fmax(m, sqrt(t / b));
     }
+  }
+  if (!END) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (l == 0) sh[w] = m;
+  double o[2] = {0.0, 0.0};
+  if (END == 1) sum_partials<2>(partials, nb, o);
+  if (END == 2) {
+    double p[1];
+    sum_partials<1>(partials, nb, p);
+    o[0] = p[0];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < KB / 32; ++i) m = fmax(m, sh[i]);
+    if (END == 1) bicgstab_end(sc, o[0], o[1], m, sg.nseg);
+    if (END == 2) gcr_end(sc, o[0], m, sg.nseg);
+    if (END == 3) *ratio = m;
   }
 }
 
@@ -325,79 +454,81 @@ __global__ void __launch_bounds__(KB) k_end_iter(KScal* sc, const double* partia
 // with the same combination applied to z, normalised, then x += alpha P,
 // r -= alpha Q with alpha = r.Q. One preconditioner application and one SpMV
 // per iteration instead of BiCGStab's two of each; the residual norm is
-// monotone.
+// monotone. Iteration k stores its direction in slot k mod 2; the first two
+// iterations find one or both slots empty and leave them out (the coefficients
+// of an empty slot are zero).
 
-// q = A z (scalar CSR); partial q.Q0, q.Q1
-template <class TM, class TV>
-__global__ void __launch_bounds__(KB) k_spmv_gcr(int nn, const int* __restrict__ rp, const int* __restrict__ cols,
-                                                  const TM* __restrict__ A, const TV* __restrict__ z,
+// q = A z; partials q.Q0, q.Q1
+template <class TM, class TV, int FORMAT>
+__global__ void __launch_bounds__(KB, 8) k_spmv_gcr(int nn, ScalarMat<TM> M, const TV* __restrict__ z,
                                                   TV* __restrict__ q, const TV* __restrict__ Q0,
                                                   const TV* __restrict__ Q1, double* partials, const KScal* sc) {
   if (sc->done) return;
+  const int have = sc->iters;
   double v[2] = {0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int k = __ldg(rp + i); k < __ldg(rp + i + 1); ++k) s += double(A[k]) * double(z[__ldg(cols + k)]);
-    const TV qs = TV(s);
+    const double q0 = have > 0 ? double(Q0[i]) : 0.0, q1 = have > 1 ? double(Q1[i]) : 0.0;
+    const TV qs = TV(scalar_row<FORMAT, TM, TV>(M, i, z));
     q[i] = qs;
-    v[0] += double(qs) * double(Q0[i]);
-    v[1] += double(qs) * double(Q1[i]);
+    v[0] += double(qs) * q0;
+    v[1] += double(qs) * q1;
   }
-  block_reduce_store<2>(v, partials, MAX_PARTIALS);
+  block_partials<2>(v, partials);
 }
 
-// beta_j = q.Q_j (d0, d1)
-__global__ void __launch_bounds__(KB) k_gcr_beta(KScal* sc, const double* partials, int nb) {
-  if (sc->done) return;
-  double o[2];
-  final_reduce<2>(partials, nb, o);
-  if (threadIdx.x == 0) {
-    sc->d0 = o[0];
-    sc->d1 = o[1];
-  }
-}
-
-// z -= beta0 P0 + beta1 P1, q -= beta0 Q0 + beta1 Q1; partial q.q, r.q
+// beta_j = q.Q_j from the product's partials, z -= beta0 P0 + beta1 P1, q -=
+// beta0 Q0 + beta1 Q1; partials q.q, r.q
 template <class TV>
-__global__ void __launch_bounds__(KB) k_gcr_orth(int n, TV* z, TV* q, const TV* P0, const TV* P1, const TV* Q0,
-                                                  const TV* Q1, const TV* r, double* partials, const KScal* sc) {
+__global__ void __launch_bounds__(KB) k_gcr_orth(int n, TV* z, TV* q, const TV* __restrict__ P0,
+                                                  const TV* __restrict__ P1, const TV* __restrict__ Q0,
+                                                  const TV* __restrict__ Q1, const TV* __restrict__ r,
+                                                  const double* __restrict__ in, int nb, double* partials,
+                                                  const KScal* sc) {
   if (sc->done) return;
-  const double b0 = sc->d0, b1 = sc->d1;
+  const int have = sc->iters;
+  double be[2];
+  sum_partials<2>(in, nb, be);
+  const double b0 = be[0], b1 = be[1];
   double v[2] = {0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    z[i] = TV(double(z[i]) - b0 * double(P0[i]) - b1 * double(P1[i]));
-    const TV qn = TV(double(q[i]) - b0 * double(Q0[i]) - b1 * double(Q1[i]));
-    q[i] = qn;
+    double zi = double(z[i]), qi = double(q[i]);
+    if (have > 0) {
+      zi -= b0 * double(P0[i]);
+      qi -= b0 * double(Q0[i]);
+    }
+    if (have > 1) {
+      zi -= b1 * double(P1[i]);
+      qi -= b1 * double(Q1[i]);
+    }
+    if (have > 0) z[i] = TV(zi);
+    const TV qn = TV(qi);
+    if (have > 0) q[i] = qn;
     v[0] += double(qn) * double(qn);
     v[1] += double(r[i]) * double(qn);
   }
-  block_reduce_store<2>(v, partials, MAX_PARTIALS);
+  block_partials<2>(v, partials);
 }
 
-// 1/|q| (omega) and alpha = r.q / |q|; a vanishing q is a breakdown
-__global__ void __launch_bounds__(KB) k_gcr_alpha(KScal* sc, const double* partials, int nb) {
-  if (sc->done) return;
-  double o[2];
-  final_reduce<2>(partials, nb, o);
-  if (threadIdx.x == 0) {
-    const double nq = sqrt(o[0]);
-    if (!(nq > 0.0) || !(nq < INFINITY)) {
-      sc->done = 1;
-      sc->status = nq < INFINITY ? 1 : 2;
-      return;
-    }
-    sc->omega = 1.0 / nq;
-    sc->alpha = o[1] / nq;
-  }
-}
-
-// P = z / |q|, Q = q / |q| into the oldest slot; x += alpha P, r -= alpha Q;
+// 1/|q| and alpha = r.q / |q| from the partials (a vanishing q is a breakdown),
+// P = z / |q|, Q = q / |q| into the oldest slot, x += alpha P, r -= alpha Q;
 // partial r.r
 template <class TV>
-__global__ void __launch_bounds__(KB) k_gcr_update(int n, TV* x, TV* r, const TV* z, const TV* q, TV* P, TV* Q,
-                                                    double* partials, const KScal* sc) {
+__global__ void __launch_bounds__(KB) k_gcr_update(int n, TV* x, TV* r, const TV* __restrict__ z,
+                                                    const TV* __restrict__ q, TV* __restrict__ P, TV* __restrict__ Q,
+                                                    const double* __restrict__ in, int nb, double* partials,
+                                                    KScal* sc) {
   if (sc->done) return;
-  const double inv = sc->omega, al = sc->alpha;
+  double o[2];
+  sum_partials<2>(in, nb, o);
+  const double nq = sqrt(o[0]);
+  if (!(nq > 0.0) || !(nq < INFINITY)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      sc->done = 1;
+      sc->status = nq < INFINITY ? 1 : 2;
+    }
+    return;
+  }
+  const double inv = 1.0 / nq, al = o[1] / nq;
   double v[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const TV pi = TV(double(z[i]) * inv), qi = TV(double(q[i]) * inv);
@@ -408,34 +539,7 @@ __global__ void __launch_bounds__(KB) k_gcr_update(int n, TV* x, TV* r, const TV
     r[i] = rn;
     v[0] += double(rn) * double(rn);
   }
-  block_reduce_store<1>(v, partials, MAX_PARTIALS);
-}
-
-// residual norm and convergence test; an iteration that leaves the residual
-// where it was (truncated GCR can stagnate when the preconditioned operator's
-// symmetric part is not definite) ends the solve with status 1, and the
-// caller falls back to BiCGStab
-__global__ void __launch_bounds__(KB) k_gcr_end(KScal* sc, const double* partials, int nb, const double* seg_r2,
-                                                 const double* seg_b2, int nseg) {
-  if (sc->done) return;
-  double o[1];
-  final_reduce<1>(partials, nb, o);
-  const double segmax = block_seg_max(seg_r2, seg_b2, nseg);
-  if (threadIdx.x == 0) {
-    sc->seg_rel = segmax;
-    const double prev = sc->rnorm;
-    sc->rnorm = sqrt(o[0]);
-    sc->iters += 1;
-    if (!(sc->rnorm < INFINITY)) {
-      sc->done = 1;
-      sc->status = 2;
-    } else if ((nseg > 1 ? segmax <= sc->rtol : sc->rnorm <= sc->rtol * sc->bnorm) || sc->iters >= sc->maxit) {
-      sc->done = 1;
-    } else if (sc->rnorm > 0.9999 * prev) {
-      sc->done = 1;
-      sc->status = 1;
-    }
-  }
+  block_partials<1>(v, partials);
 }
 
 // ---------------------------------------------------------------------------
@@ -451,7 +555,7 @@ int KrylovSolver<B, TM, TV>::setup(int nn_, const int* rp_, const int* cols_, co
   const size_t n = (size_t)B * nn;
   for (int k = 0; k < 8; ++k) OA_CUDA(cudaMalloc(&vec[k], sizeof(TV) * n));
   OA_CUDA(cudaMalloc(&Minv, sizeof(double) * (size_t)B * B * nn));
-  OA_CUDA(cudaMalloc(&partials, sizeof(double) * 3 * MAX_PARTIALS));
+  OA_CUDA(cudaMalloc(&partials, sizeof(double) * partials_size()));
   OA_CUDA(cudaMalloc(&scal, sizeof(KScal)));
   OA_CUDA(cudaMallocHost(&hscal, sizeof(KScal)));
   return OA_OK;
@@ -461,7 +565,7 @@ template <int B, class TM, class TV>
 size_t KrylovSolver<B, TM, TV>::storage_bytes(int nn_) {
   const size_t n = (size_t)B * nn_;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  return 8 * up(sizeof(TV) * n) + up(sizeof(double) * (size_t)B * B * nn_) + up(sizeof(double) * 3 * MAX_PARTIALS) +
+  return 8 * up(sizeof(TV) * n) + up(sizeof(double) * (size_t)B * B * nn_) + up(sizeof(double) * partials_size()) +
          up(sizeof(KScal));
 }
 
@@ -486,7 +590,7 @@ int KrylovSolver<B, TM, TV>::attach(int nn_, const int* rp_, const int* cols_, c
   Minv = reinterpret_cast<double*>(p);
   p += up(sizeof(double) * (size_t)B * B * nn);
   partials = reinterpret_cast<double*>(p);
-  p += up(sizeof(double) * 3 * MAX_PARTIALS);
+  p += up(sizeof(double) * partials_size());
   scal = p;
   return OA_OK;
 }
@@ -516,42 +620,39 @@ void KrylovSolver<B, TM, TV>::release() {
 }
 
 template <int B, class TM, class TV>
+bool KrylovSolver<B, TM, TV>::uses_amg() const {
+  return B == 1 && std::is_same<TM, TV>::value && amg != nullptr;
+}
+
+template <int B, class TM, class TV>
 int KrylovSolver<B, TM, TV>::precond(const TV* in, TV* out) {
-  constexpr bool kAmgOk = (B == 1) && std::is_same<TM, TV>::value;
-  KScal* sc = static_cast<KScal*>(scal);
-  if constexpr (kAmgOk) {
-    if (amg) return amg->apply(reinterpret_cast<const TV*>(in), out, &sc->done, st);
-  }
-  const int gfull = (B * nn + KB - 1) / KB;
-  k_prec<B, TV><<<gfull, KB, 0, st>>>(nn, reinterpret_cast<const TV*>(Minv), in, out, sc);
-  count_launches(1);
+  if constexpr (B == 1 && std::is_same<TM, TV>::value)
+    if (amg) return amg->apply(in, out, &static_cast<KScal*>(scal)->done, st);
   return OA_OK;
 }
 
-// x = 0, r = rh = b, p = v = 0, inverse (block) diagonal, device scalars; the
-// GCR(2) direction slots start at zero (no stored directions yet)
+// x = 0, r = b (rh = b), the inverse (block) diagonal of the Jacobi
+// preconditioner, device scalars
 template <int B, class TM, class TV>
 template <class TB>
 int KrylovSolver<B, TM, TV>::prologue(const TM* A, const TB* b, double rtol, int maxit, const double* rtol_dev,
                                       const int* maxit_dev, bool use_gcr) {
   const int n = B * nn;
-  TV *x = static_cast<TV*>(vec[0]), *r = static_cast<TV*>(vec[1]), *rh = static_cast<TV*>(vec[2]),
-     *p = static_cast<TV*>(vec[3]), *v = static_cast<TV*>(vec[4]);
   KScal* sc = static_cast<KScal*>(scal);
-  const int gfull = (n + KB - 1) / KB;
-  const int gv = gfull < MAX_PARTIALS ? gfull : MAX_PARTIALS;
-  const int gr = (nn + KB - 1) / KB;
-  k_build_minv<B, TM, TV><<<gr, KB, 0, st>>>(nn, rp, dg, A, reinterpret_cast<TV*>(Minv));
-  k_init<TV, TB><<<gv, KB, 0, st>>>(n, b, x, r, rh, p, v, partials);
+  const int gv = reduce_grid(n);
+  if (!uses_amg()) {
+    k_build_minv<B, TM, TV><<<(nn + KB - 1) / KB, KB, 0, st>>>(nn, rp, dg, A, reinterpret_cast<TV*>(Minv));
+    count_launches(1);
+  }
+  k_init<TV, TB><<<gv, KB, 0, st>>>(n, b, static_cast<TV*>(vec[0]), static_cast<TV*>(vec[1]),
+                                    use_gcr ? nullptr : static_cast<TV*>(vec[2]), partials);
   k_init_scalars<<<1, KB, 0, st>>>(sc, partials, gv, rtol, maxit, rtol_dev, maxit_dev);
-  count_launches(3);
+  count_launches(2);
   if (seg.on()) {
-    k_seg_sumsq<TB><<<seg.nseg, KB, 0, st>>>(seg.ptr, seg.rows, b, seg.b2, nullptr);
+    k_segments<TB, 0><<<seg.nchunk, KB, 0, st>>>(seg, b, seg.b2, nullptr, nullptr, nullptr, nullptr, 0);
     count_launches(1);
   }
   OA_CUDA(cudaGetLastError());
-  if (use_gcr)
-    for (int k = 4; k < 8; ++k) OA_CUDA(cudaMemsetAsync(vec[k], 0, sizeof(TV) * (size_t)n, st));
   return OA_OK;
 }
 
@@ -564,46 +665,51 @@ int KrylovSolver<B, TM, TV>::chunk(const TM* A, int check_every, bool use_gcr) {
      *p = static_cast<TV*>(vec[3]), *v = static_cast<TV*>(vec[4]), *ph = static_cast<TV*>(vec[5]),
      *sh = static_cast<TV*>(vec[6]), *t = static_cast<TV*>(vec[7]);
   KScal* sc = static_cast<KScal*>(scal);
-  const int gfull = (n + KB - 1) / KB;
-  const int gv = gfull < MAX_PARTIALS ? gfull : MAX_PARTIALS;
+  const int gv = reduce_grid(n);
+  // two sets of partials: a kernel reads the one and writes the other
+  double *pa = partials, *pb = partials + 2 * MAX_PARTIALS;
+  const ScalarMat<TM> M = {rp, cols, A, ell.cols, static_cast<const TM*>(ell_val)};
+  const int format = B == 1 && ell_val ? ell_format(ell.w, ell.slots, sizeof(TM)) : 1;
   if (use_gcr) {
     // GCR(2) work vectors in the same buffers: x r z q P0 P1 Q0 Q1
     TV *gz = rh, *gq = p, *gP[2] = {v, ph}, *gQ[2] = {sh, t};
     for (int it = 0; it < check_every; ++it) {
       const int slot = it & 1;  // the older of the two stored directions
       if (int s = precond(r, gz)) return s;
-      k_spmv_gcr<TM, TV><<<gv, KB, 0, st>>>(nn, rp, cols, A, gz, gq, gQ[0], gQ[1], partials, sc);
-      k_gcr_beta<<<1, KB, 0, st>>>(sc, partials, gv);
-      k_gcr_orth<TV><<<gv, KB, 0, st>>>(n, gz, gq, gP[0], gP[1], gQ[0], gQ[1], r, partials, sc);
-      k_gcr_alpha<<<1, KB, 0, st>>>(sc, partials, gv);
-      k_gcr_update<TV><<<gv, KB, 0, st>>>(n, x, r, gz, gq, gP[slot], gQ[slot], partials, sc);
-      if (seg.on()) {
-        k_seg_sumsq<TV><<<seg.nseg, KB, 0, st>>>(seg.ptr, seg.rows, r, seg.r2, &sc->done);
-        count_launches(1);
-      }
-      k_gcr_end<<<1, KB, 0, st>>>(sc, partials, gv, seg.r2, seg.b2, seg.on() ? seg.nseg : 0);
+#define OA_CALL(F) k_spmv_gcr<TM, TV, F><<<gv, KB, 0, st>>>(nn, M, gz, gq, gQ[0], gQ[1], pa, sc)
+      OA_FORMAT(format, OA_CALL)
+#undef OA_CALL
+      k_gcr_orth<TV><<<gv, KB, 0, st>>>(n, gz, gq, gP[0], gP[1], gQ[0], gQ[1], r, pa, gv, pb, sc);
+      k_gcr_update<TV><<<gv, KB, 0, st>>>(n, x, r, gz, gq, gP[slot], gQ[slot], pb, gv, pa, sc);
+      if (seg.on())
+        k_segments<TV, 2><<<seg.nchunk, KB, 0, st>>>(seg, r, seg.r2, seg.b2, sc, nullptr, pa, gv);
+      else
+        k_end_iter<true><<<1, KB, 0, st>>>(sc, pa, gv);
+      count_launches(4);
     }
-    count_launches(6L * check_every);
     OA_CUDA(cudaGetLastError());
     return OA_OK;
   }
+  const TV* Mi = uses_amg() ? nullptr : reinterpret_cast<const TV*>(Minv);
+  const int gr = (nn + KB - 1) / KB;
   for (int it = 0; it < check_every; ++it) {
-    k_p_update<TV><<<gfull, KB, 0, st>>>(n, p, r, v, sc);
+    k_p_update<B, TV><<<gr, KB, 0, st>>>(nn, p, r, v, Mi, ph, sc);
     if (int s = precond(p, ph)) return s;
-    k_spmv<B, TM, TV, 1><<<gv, KB, 0, st>>>(nn, rp, cols, A, ph, v, rh, nullptr, partials, sc);
-    k_alpha<<<1, KB, 0, st>>>(sc, partials, gv);
-    k_s_update<TV><<<gfull, KB, 0, st>>>(n, r, v, sc);
+#define OA_CALL(F) k_spmv<B, TM, TV, 1, B == 1 ? F : 1><<<gv, KB, 0, st>>>(nn, M, ph, v, rh, pa, sc)
+    OA_FORMAT(format, OA_CALL)
+#undef OA_CALL
+    k_s_update<B, TV><<<reduce_grid(nn), KB, 0, st>>>(nn, r, v, Mi, sh, pa, gv, sc);
     if (int s = precond(r, sh)) return s;
-    k_spmv<B, TM, TV, 2><<<gv, KB, 0, st>>>(nn, rp, cols, A, sh, t, r, nullptr, partials, sc);
-    k_omega<<<1, KB, 0, st>>>(sc, partials, gv);
-    k_x_update<TV><<<gv, KB, 0, st>>>(n, x, r, ph, sh, t, rh, partials, sc);
-    if (seg.on()) {
-      k_seg_sumsq<TV><<<seg.nseg, KB, 0, st>>>(seg.ptr, seg.rows, r, seg.r2, &sc->done);
-      count_launches(1);
-    }
-    k_end_iter<<<1, KB, 0, st>>>(sc, partials, gv, seg.r2, seg.b2, seg.on() ? seg.nseg : 0);
+#define OA_CALL(F) k_spmv<B, TM, TV, 2, B == 1 ? F : 1><<<gv, KB, 0, st>>>(nn, M, sh, t, r, pb, sc)
+    OA_FORMAT(format, OA_CALL)
+#undef OA_CALL
+    k_x_update<TV><<<gv, KB, 0, st>>>(n, x, r, ph, sh, t, rh, pb, gv, pa, sc);
+    if (seg.on())
+      k_segments<TV, 1><<<seg.nchunk, KB, 0, st>>>(seg, r, seg.r2, seg.b2, sc, nullptr, pa, gv);
+    else
+      k_end_iter<false><<<1, KB, 0, st>>>(sc, pa, gv);
+    count_launches(6);
   }
-  count_launches(8L * check_every);
   OA_CUDA(cudaGetLastError());
   return OA_OK;
 }
@@ -734,28 +840,82 @@ OA_EMIT(3, float, float, float)
 #undef OA_EMIT
 
 // ---------------------------------------------------------------------------
+// fixed-width storage
+__global__ void k_ell_cols(int n, int w, const int* rp, const int* cols, int* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (n + 31) / 32 * 32) return;
+  const int a = i < n ? rp[i] : 0, len = i < n ? rp[i + 1] - a : 0, pad = len ? cols[a] : 0;
+  for (int q = 0; q < w; ++q) out[(size_t)(i >> 5) * 32 * w + 32 * q + (i & 31)] = q < len ? cols[a + q] : pad;
+}
+
+template <class T, int W>
+__global__ void __launch_bounds__(256) k_ell_values(int n, const int* __restrict__ rp, const T* __restrict__ csr,
+                                                    T* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (n + 31) / 32 * 32) return;
+  const int a = i < n ? __ldg(rp + i) : 0, len = i < n ? __ldg(rp + i + 1) - a : 0;
+  T v[W];
+#pragma unroll
+  for (int q = 0; q < W; ++q) v[q] = q < len ? __ldg(csr + a + q) : T(0);
+#pragma unroll
+  for (int q = 0; q < W; ++q) out[(size_t)(i >> 5) * 32 * W + 32 * q + (i & 31)] = v[q];
+}
+
+int ell_graph(int n, const int* h_rp, const int* rp, const int* cols, EllGraph* out, cudaStream_t st) {
+  *out = EllGraph{};
+  int longest = 0;
+  for (int i = 0; i < n; ++i) longest = std::max(longest, h_rp[i + 1] - h_rp[i]);
+  const int w = longest <= 7 ? 7 : 15;
+  const long long slots = (n + 31LL) / 32 * 32 * w;
+  if (longest > w || slots > 2LL * h_rp[n] + 4096) return OA_OK;
+  int* c = nullptr;
+  if (cudaMalloc(&c, sizeof(int) * slots) != cudaSuccess)
+    return fail(OA_ERR_CUDA, "fixed-width matrix storage: allocation failed");
+  out->w = w;
+  out->cols = c;
+  out->slots = slots;
+  k_ell_cols<<<(n + 31) / 32 * 32 / 32, 32, 0, st>>>(n, w, rp, cols, c);
+  count_launches(1);
+  OA_CUDA(cudaGetLastError());
+  return OA_OK;
+}
+
+template <class T>
+int ell_values(int n, const int* rp, const T* csr, int w, T* out, cudaStream_t st) {
+  const int g = ((n + 31) / 32 * 32 + 255) / 256;
+  if (w == 7) k_ell_values<T, 7><<<g, 256, 0, st>>>(n, rp, csr, out);
+  else k_ell_values<T, 15><<<g, 256, 0, st>>>(n, rp, csr, out);
+  count_launches(1);
+  OA_CUDA(cudaGetLastError());
+  return OA_OK;
+}
+template int ell_values<float>(int, const int*, const float*, int, float*, cudaStream_t);
+template int ell_values<double>(int, const int*, const double*, int, double*, cudaStream_t);
+
+// ---------------------------------------------------------------------------
 // FP64 residual for iterative refinement: r = b - A x (A in its stored
 // precision, arithmetic in FP64), with partial ||r||^2.
-template <class TM>
-__global__ void __launch_bounds__(KB) k_residual(int nn, const int* __restrict__ rp, const int* __restrict__ cols,
-                                                  const TM* __restrict__ A, const double* __restrict__ x,
+template <class TM, int FORMAT>
+__global__ void __launch_bounds__(KB) k_residual(int nn, ScalarMat<TM> M, const double* __restrict__ x,
                                                   const double* __restrict__ b, double* __restrict__ r,
                                                   double* partials) {
   double v[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k) s += double(A[k]) * x[cols[k]];
-    const double ri = b[i] - s;
+    const double bi = b[i];
+    const double ri = bi - scalar_row<FORMAT, TM, double>(M, i, x);
     r[i] = ri;
     v[0] += ri * ri;
   }
-  block_reduce_store<1>(v, partials, MAX_PARTIALS);
+  block_partials<1>(v, partials);
 }
 
-__global__ void __launch_bounds__(KB) k_norm_out(const double* partials, int nb, double* out) {
-  double o[1];
-  final_reduce<1>(partials, nb, o);
-  if (threadIdx.x == 0) *out = sqrt(o[0]);
+template <bool ROOT, int NV>
+__global__ void __launch_bounds__(KB) k_sums_out(const double* partials, int nb, double* out) {
+  double o[NV];
+  sum_partials<NV>(partials, nb, o);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) out[k] = ROOT ? sqrt(o[k]) : o[k];
 }
 
 template <class TV>
@@ -765,77 +925,63 @@ __global__ void k_add_correction(int n, double* x, const TV* d) {
 }
 
 template <class TM>
-int fp64_residual(int nn, const int* rp, const int* cols, const TM* A, const double* x, const double* b, double* r,
-                  double* partials, double* norm_dev, cudaStream_t st) {
-  const int gf = (nn + KB - 1) / KB;
-  const int g = gf < MAX_PARTIALS ? gf : MAX_PARTIALS;
-  k_residual<TM><<<g, KB, 0, st>>>(nn, rp, cols, A, x, b, r, partials);
-  k_norm_out<<<1, KB, 0, st>>>(partials, g, norm_dev);
+int KrylovMatrix<TM>::residual(int nn, const double* x, const double* b, double* r, double* partials,
+                               double* norm_dev, cudaStream_t st) const {
+  const int g = reduce_grid(nn);
+  const ScalarMat<TM> M = {rp, cols, A, ell.cols, eval};
+#define OA_CALL(F) k_residual<TM, F><<<g, KB, 0, st>>>(nn, M, x, b, r, partials)
+  OA_FORMAT(eval ? ell_format(ell.w, ell.slots, sizeof(TM)) : 1, OA_CALL)
+#undef OA_CALL
+  k_sums_out<true, 1><<<1, KB, 0, st>>>(partials, g, norm_dev);
   count_launches(2);
   OA_CUDA(cudaGetLastError());
   return OA_OK;
 }
-template int fp64_residual<float>(int, const int*, const int*, const float*, const double*, const double*, double*,
-                                  double*, double*, cudaStream_t);
-template int fp64_residual<double>(int, const int*, const int*, const double*, const double*, const double*, double*,
-                                   double*, double*, cudaStream_t);
+template struct KrylovMatrix<float>;
 
-__global__ void __launch_bounds__(KB) k_sumsq_partial(int n, const double* __restrict__ v, double* partials) {
+__global__ void __launch_bounds__(KB) k_sumsq(int n, const double* __restrict__ v, double* partials) {
   double s[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s[0] += v[i] * v[i];
-  block_reduce_store<1>(s, partials, MAX_PARTIALS);
-}
-
-__global__ void __launch_bounds__(KB) k_sum_out(const double* partials, int nb, double* out) {
-  double o[1];
-  final_reduce<1>(partials, nb, o);
-  if (threadIdx.x == 0) *out = o[0];
+  block_partials<1>(s, partials);
 }
 
 int device_sumsq(int n, const double* v, double* out, double* partials, cudaStream_t st) {
-  const int gf = (n + KB - 1) / KB;
-  const int g = gf < MAX_PARTIALS ? gf : MAX_PARTIALS;
-  k_sumsq_partial<<<g, KB, 0, st>>>(n, v, partials);
-  k_sum_out<<<1, KB, 0, st>>>(partials, g, out);
+  const int g = reduce_grid(n);
+  k_sumsq<<<g, KB, 0, st>>>(n, v, partials);
+  k_sums_out<false, 1><<<1, KB, 0, st>>>(partials, g, out);
   count_launches(2);
   OA_CUDA(cudaGetLastError());
   return OA_OK;
 }
 
-int partials_size() { return 3 * MAX_PARTIALS; }
+int partials_size() { return 6 * MAX_PARTIALS; }
 
-// per-component sums of squares of a [nn][3] vector (ordered two-stage tree)
+// per-component sums of squares of two [nn][3] vectors
 template <class T>
-__global__ void __launch_bounds__(KB) k_comp_sumsq3(int nn, const T* __restrict__ v, double* partials) {
-  double s[3] = {0.0, 0.0, 0.0};
+__global__ void __launch_bounds__(KB) k_comp_sumsq3(int nn, const T* __restrict__ a, const T* __restrict__ b,
+                                                     double* partials) {
+  double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x)
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const double a = double(v[3 * (size_t)i + k]);
-      s[k] += a * a;
+      const double p = double(a[3 * (size_t)i + k]), q = double(b[3 * (size_t)i + k]);
+      s[k] += p * p;
+      s[3 + k] += q * q;
     }
-  block_reduce_store<3>(s, partials, MAX_PARTIALS);
-}
-
-__global__ void __launch_bounds__(KB) k_sum3_out(const double* partials, int nb, double* out) {
-  double o[3];
-  final_reduce<3>(partials, nb, o);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; ++k) out[k] = o[k];
+  block_partials<6>(s, partials);
 }
 
 template <class T>
-int device_comp_sumsq3(int nn, const T* v, double* out, double* partials, cudaStream_t st) {
-  const int gf = (nn + KB - 1) / KB;
-  const int g = gf < MAX_PARTIALS ? gf : MAX_PARTIALS;
-  k_comp_sumsq3<T><<<g, KB, 0, st>>>(nn, v, partials);
-  k_sum3_out<<<1, KB, 0, st>>>(partials, g, out);
+int device_comp_sumsq3(int nn, const T* a, const T* b, double* out, double* partials, cudaStream_t st) {
+  const int g = reduce_grid(nn);
+  k_comp_sumsq3<T><<<g, KB, 0, st>>>(nn, a, b, partials);
+  k_sums_out<false, 6><<<1, KB, 0, st>>>(partials, g, out);
   count_launches(2);
   OA_CUDA(cudaGetLastError());
   return OA_OK;
 }
-template int device_comp_sumsq3<float>(int, const float*, double*, double*, cudaStream_t);
-template int device_comp_sumsq3<double>(int, const double*, double*, double*, cudaStream_t);
+template int device_comp_sumsq3<float>(int, const float*, const float*, double*, double*, cudaStream_t);
+template int device_comp_sumsq3<double>(int, const double*, const double*, double*, double*, cudaStream_t);
 
 template <class TV>
 int add_correction(int n, double* x, const TV* d, cudaStream_t st) {
@@ -850,7 +996,7 @@ template int add_correction<double>(int, double*, const double*, cudaStream_t);
 template <class T>
 int segment_sumsq(const Segments& sg, const T* v, double* out, cudaStream_t st) {
   if (!sg.on()) return OA_OK;
-  k_seg_sumsq<T><<<sg.nseg, KB, 0, st>>>(sg.ptr, sg.rows, v, out, nullptr);
+  k_segments<T, 0><<<sg.nchunk, KB, 0, st>>>(sg, v, out, nullptr, nullptr, nullptr, nullptr, 0);
   count_launches(1);
   OA_CUDA(cudaGetLastError());
   return OA_OK;
@@ -858,8 +1004,8 @@ int segment_sumsq(const Segments& sg, const T* v, double* out, cudaStream_t st) 
 template int segment_sumsq<float>(const Segments&, const float*, double*, cudaStream_t);
 template int segment_sumsq<double>(const Segments&, const double*, double*, cudaStream_t);
 
-int segment_max_ratio(const Segments& sg, double* out, cudaStream_t st) {
-  k_seg_max_ratio<<<1, KB, 0, st>>>(sg.r2, sg.b2, sg.nseg, out);
+int segment_ratio(const Segments& sg, const double* v, double* out, cudaStream_t st) {
+  k_segments<double, 3><<<sg.nchunk, KB, 0, st>>>(sg, v, sg.r2, sg.b2, nullptr, out, nullptr, 0);
   count_launches(1);
   OA_CUDA(cudaGetLastError());
   return OA_OK;

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "oa_amg.h"
+#include "oa_ell.cuh"
 #include "oa_graph.h"
 
 namespace oa {
@@ -18,24 +19,29 @@ struct KScal {
 };
 
 // Independent systems solved as one (a batch of disjoint meshes): the rows of
-// each segment (seg_rows[seg_ptr[s] .. seg_ptr[s+1])) and scratch for the
+// all segments, segment after segment, cut into chunks that each lie in one
+// segment (chunk c: rows[chunk[c] .. chunk[c + 1]), segment s: chunks
+// chunk_ptr[s] .. chunk_ptr[s + 1]), and scratch for the chunks' sums and the
 // per-segment sums of squares of b and r. With nseg > 1 a solve has converged
 // when every segment's ||r_s|| <= rtol ||b_s||, not when the whole batch's
 // norm is.
 struct Segments {
-  int nseg = 0;
-  const int* ptr = nullptr;
+  int nseg = 0, nchunk = 0;
   const int* rows = nullptr;
+  const int* chunk = nullptr;      // [nchunk + 1]
+  const int* chunk_ptr = nullptr;  // [nseg + 1]
+  double* part = nullptr;          // [nchunk]
+  unsigned* ticket = nullptr;
   double* b2 = nullptr;  // [nseg]
   double* r2 = nullptr;  // [nseg]
   bool on() const { return nseg > 1; }
 };
-// per-segment sums of squares of v into out[nseg] (one block per segment,
-// fixed order)
+// per-segment sums of squares of v into out[nseg] (fixed order)
 template <class T>
 int segment_sumsq(const Segments& sg, const T* v, double* out, cudaStream_t st);
-// largest sqrt(r2[s] / b2[s]) over segments (0 where b2 = 0) into *out
-int segment_max_ratio(const Segments& sg, double* out, cudaStream_t st);
+// per-segment sums of squares of v into sg.r2 and the largest sqrt(r2[s] /
+// b2[s]) over segments (0 where b2 = 0) into *out
+int segment_ratio(const Segments& sg, const double* v, double* out, cudaStream_t st);
 
 // BiCGStab on a BSR matrix with BxB blocks; matrix values TM, vectors TV.
 template <int B, class TM, class TV>
@@ -61,6 +67,10 @@ struct KrylovSolver {
   bool graph_gcr = false;
   long long graph_launches = 0;
 
+  // the matrix in fixed-width storage (scalar systems whose caller keeps it;
+  // null: the CSR arrays are used)
+  EllGraph ell;
+  const void* ell_val = nullptr;
   // per-segment convergence (batched disjoint systems); off by default
   Segments seg;
   // storage carved from caller memory instead of cudaMalloc (no allocation)
@@ -101,6 +111,7 @@ struct KrylovSolver {
   TV* solution() const { return static_cast<TV*>(vec[0]); }
 
  private:
+  bool uses_amg() const;
   int precond(const TV* in, TV* out);
   template <class TB>
   int prologue(const TM* A, const TB* b, double rtol, int maxit, const double* rtol_dev, const int* maxit_dev,
@@ -108,19 +119,27 @@ struct KrylovSolver {
   int chunk(const TM* A, int check_every, bool use_gcr);
 };
 
-// r = b - A x in FP64 arithmetic (A scalar CSR in its stored precision);
-// ||r|| written to norm_dev.
+// A scalar matrix as CSR and, when eval is given, in fixed-width storage.
 template <class TM>
-int fp64_residual(int nn, const int* rp, const int* cols, const TM* A, const double* x, const double* b, double* r,
-                  double* partials, double* norm_dev, cudaStream_t st);
+struct KrylovMatrix {
+  const int *rp = nullptr, *cols = nullptr;
+  const TM* A = nullptr;
+  EllGraph ell;
+  const TM* eval = nullptr;
+  // r = b - A x in FP64 arithmetic (A in its stored precision); ||r|| written to norm_dev
+  int residual(int nn, const double* x, const double* b, double* r, double* partials, double* norm_dev,
+               cudaStream_t st) const;
+};
 template <class TV>
 int add_correction(int n, double* x, const TV* d, cudaStream_t st);
 // sum of squares of v into *out (device), ordered two-stage reduction;
 // partials must hold partials_size() doubles
 int device_sumsq(int n, const double* v, double* out, double* partials, cudaStream_t st);
-// per-component sums of squares of a [nn][3] vector into out[3] (device)
+// per-component sums of squares of the [nn][3] vectors a and b into out[0..2]
+// and out[3..5] (device)
 template <class T>
-int device_comp_sumsq3(int nn, const T* v, double* out, double* partials, cudaStream_t st);
+int device_comp_sumsq3(int nn, const T* a, const T* b, double* out, double* partials, cudaStream_t st);
+// doubles of a reduction's partials buffer
 int partials_size();
 
 }  // namespace oa

@@ -150,15 +150,22 @@ __global__ void k_ir_next(cudaGraphConditionalHandle h, ScalarGraphState* S, Bod
 }
 }  // namespace
 
-int ScalarSolve::init(int nn) {
+int ScalarSolve::init(const ScalarGraph& g, bool mixed) {
+  const int nn = g.nn;
   if (const char* e = std::getenv("OA_AMG_REFRESH")) refresh = std::max(1, std::atoi(e));
   if (const char* e = std::getenv("OA_AMG_DRIFT")) drift_max = std::atof(e);
   if (const char* e = std::getenv("OA_IR_INNER")) inner_floor = std::atof(e);
   if (const char* e = std::getenv("OA_KRYLOV")) gcr = std::strcmp(e, "bicgstab") != 0;
   if (const char* e = std::getenv("OA_GCR_CHUNK")) gcr_chunk = std::max(2, std::atoi(e) / 2 * 2);
-  if (n == nn && r) return OA_OK;
+  const size_t ell_bytes = (mixed ? sizeof(float) : sizeof(double)) * (size_t)std::max<long long>(1, g.ell.slots);
+  if (n == nn && r && ell_size >= ell_bytes) return OA_OK;
   release();
   n = nn;
+  if (cudaMalloc(&ell, ell_bytes) != cudaSuccess) {
+    release();
+    return fail(OA_ERR_CUDA, "scalar solve: device allocation failed");
+  }
+  ell_size = ell_bytes;
   if (cudaMalloc(&r, sizeof(double) * (nn ? nn : 1)) != cudaSuccess ||
       cudaMalloc(&r32, sizeof(float) * (nn ? nn : 1)) != cudaSuccess ||
       cudaMalloc(&scal, sizeof(double) * 2) != cudaSuccess ||
@@ -173,21 +180,55 @@ int ScalarSolve::init(int nn) {
   return OA_OK;
 }
 
+// Values of the system's matrix in fixed-width storage: once per solve, for all
+// its products and the finest level's smoothing (25 us at 2.1M rows in FP32,
+// where each of the 60 passes over the matrix saves about 10).
+int ScalarSolve::widen_matrix(const ScalarGraph& g, bool mixed, const void* A, cudaStream_t st) {
+  const bool on = g.ell.w != 0;
+  k64.ell = k32.ell = g.ell;
+  k64.ell_val = on && !mixed ? ell : nullptr;
+  k32.ell_val = on && mixed ? ell : nullptr;
+  amg64.set_finest(g.ell, static_cast<const double*>(k64.ell_val));
+  amg32.set_finest(g.ell, static_cast<const float*>(k32.ell_val));
+  if (!on) return OA_OK;
+  return mixed ? ell_values<float>(g.nn, g.rp, static_cast<const float*>(A), g.ell.w, static_cast<float*>(ell), st)
+               : ell_values<double>(g.nn, g.rp, static_cast<const double*>(A), g.ell.w, static_cast<double*>(ell), st);
+}
+
 int ScalarSolve::set_segments(const std::vector<int>& ptr, const std::vector<int>& rows) {
   release_segments();
   const int nseg = (int)ptr.size() - 1;
   if (nseg <= 1) return OA_OK;
-  if (cudaMalloc(&seg_dev, sizeof(int) * (ptr.size() + rows.size())) != cudaSuccess ||
-      cudaMalloc(&seg_buf, sizeof(double) * 4 * nseg) != cudaSuccess ||
+  // chunks of at most SEG_CHUNK rows, so that a few large segments still fill
+  // the GPU (with a block per segment a batch of 16 cavities took 33 us per
+  // Krylov iteration for its sums)
+  constexpr int SEG_CHUNK = 4096;
+  std::vector<int> chunk(1, 0), cptr(1, 0);
+  for (int s = 0; s < nseg; ++s) {
+    const int len = ptr[s + 1] - ptr[s], parts = std::max(1, (len + SEG_CHUNK - 1) / SEG_CHUNK);
+    for (int c = 1; c <= parts; ++c) chunk.push_back(ptr[s] + (int)((long long)len * c / parts));
+    cptr.push_back((int)chunk.size() - 1);
+  }
+  const int nchunk = (int)chunk.size() - 1;
+  std::vector<int> all(chunk);
+  all.insert(all.end(), cptr.begin(), cptr.end());
+  all.insert(all.end(), rows.begin(), rows.end());
+  all.push_back(0);  // the ticket
+  if (cudaMalloc(&seg_dev, sizeof(int) * all.size()) != cudaSuccess ||
+      cudaMalloc(&seg_buf, sizeof(double) * (4 * nseg + nchunk)) != cudaSuccess ||
       cudaMalloc(&seg_rel, sizeof(double)) != cudaSuccess) {
     release_segments();
     return fail(OA_ERR_CUDA, "scalar solve: segment allocation failed");
   }
-  OA_CUDA(cudaMemcpy(seg_dev, ptr.data(), sizeof(int) * ptr.size(), cudaMemcpyHostToDevice));
-  OA_CUDA(cudaMemcpy(seg_dev + ptr.size(), rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice));
-  seg_in.nseg = seg_out.nseg = nseg;
-  seg_in.ptr = seg_out.ptr = seg_dev;
-  seg_in.rows = seg_out.rows = seg_dev + ptr.size();
+  OA_CUDA(cudaMemcpy(seg_dev, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice));
+  seg_in.nseg = nseg;
+  seg_in.nchunk = nchunk;
+  seg_in.chunk = seg_dev;
+  seg_in.chunk_ptr = seg_dev + chunk.size();
+  seg_in.rows = seg_in.chunk_ptr + cptr.size();
+  seg_in.ticket = reinterpret_cast<unsigned*>(seg_dev + all.size() - 1);
+  seg_in.part = seg_buf + 4 * nseg;
+  seg_out = seg_in;
   seg_in.b2 = seg_buf;
   seg_in.r2 = seg_buf + nseg;
   seg_out.b2 = seg_buf + 2 * nseg;
@@ -221,6 +262,9 @@ void ScalarSolve::release() {
   diag_ref = nullptr;
   drift = nullptr;
   hdrift = nullptr;
+  if (ell) cudaFree(ell);
+  ell = nullptr;
+  ell_size = 0;
   if (r) cudaFree(r);
   if (r32) cudaFree(r32);
   if (scal) cudaFree(scal);
@@ -241,7 +285,7 @@ void ScalarSolve::release() {
 int ScalarSolve::solve(const ScalarGraph& g, bool mixed, bool amg, bool graphs, const void* A, const double* b,
                        double* x, double rtol, int maxit, int* iters, double* res, int* refinements, cudaStream_t st,
                        const char* what) {
-  if (int s = init(g.nn)) return s;
+  if (int s = init(g, mixed)) return s;
   if (amg) {
     if (!mixed && !amg64.ready)
       if (int s = amg64.setup(g.nn, g.h_rp, g.h_cols, g.h_diag, g.rp, g.cols, g.diag)) return s;
@@ -274,6 +318,7 @@ int ScalarSolve::solve(const ScalarGraph& g, bool mixed, bool amg, bool graphs, 
   }
   if (amg && !reuse)
     if (int s = mixed ? launch_store<float>(g, A, diag_ref, st) : launch_store<double>(g, A, diag_ref, st)) return s;
+  if (int s = widen_matrix(g, mixed, A, st)) return s;
   if (!mixed) {
     if (int s = k64.setup(g.nn, g.rp, g.cols, g.diag, st)) return s;
     double* xs = nullptr;
@@ -332,12 +377,11 @@ int ScalarSolve::solve(const ScalarGraph& g, bool mixed, bool amg, bool graphs, 
     // a diverged inner solve contributes nothing; the next pass restarts from
     // the FP64 residual
     if (k32.last_status != 3 && r_in < 1.0) add_correction<float>(g.nn, x, d, st);
-    if (int s = fp64_residual<float>(g.nn, g.rp, g.cols, A32, x, b, r, k32.partials, scal + 1, st)) return s;
+    if (int s = matrix32(g, A32).residual(g.nn, x, b, r, k32.partials, scal + 1, st)) return s;
     OA_CUDA(cudaMemcpyAsync(hscal + 1, scal + 1, sizeof(double), cudaMemcpyDeviceToHost, st));
     if (seg_out.on()) {
       // batched disjoint systems: the worst segment's relative residual
-      if (int s = segment_sumsq<double>(seg_out, r, seg_out.r2, st)) return s;
-      if (int s = segment_max_ratio(seg_out, seg_rel, st)) return s;
+      if (int s = segment_ratio(seg_out, r, seg_rel, st)) return s;
       OA_CUDA(cudaMemcpyAsync(hscal, seg_rel, sizeof(double), cudaMemcpyDeviceToHost, st));
     }
     OA_CUDA(cudaStreamSynchronize(st));
@@ -358,7 +402,7 @@ int ScalarSolve::solve(const ScalarGraph& g, bool mixed, bool amg, bool graphs, 
 
 int ScalarSolve::emit(GraphBuild& gb, cudaGraph_t g, Deps& d, const ScalarGraph& gr, bool mixed, bool amg,
                       const void* A, const double* b, double* x, double rtol, int maxit, cudaStream_t st) {
-  if (int s = init(gr.nn)) return s;
+  if (int s = init(gr, mixed)) return s;
   if (amg && !(mixed ? amg32.ready : amg64.ready))
     return fail(OA_ERR_NOT_READY, "scalar solve graph: the preconditioner is set up by a first eager solve");
   if (!gs) {
@@ -378,6 +422,7 @@ int ScalarSolve::emit(GraphBuild& gb, cudaGraph_t g, Deps& d, const ScalarGraph&
   }
   const bool use_gcr = amg && gcr;
   const int chunk_gcr = gcr_chunk;
+  if (int s = gb.seg(g, d, -1, [&]() -> int { return widen_matrix(gr, mixed, A, st); })) return s;
   // AMG numeric phase under the refresh IF
   if (amg) {
     cudaGraphConditionalHandle hn;
@@ -491,11 +536,9 @@ int ScalarSolve::emit(GraphBuild& gb, cudaGraph_t g, Deps& d, const ScalarGraph&
         k_ir_after<<<1, 1, 0, st>>>(gs, k32.scalars());
         k_add_correction_if<float><<<(gr.nn + 255) / 256, 256, 0, st>>>(gr.nn, x, k32.solution(), gs);
         count_launches(2);
-        if (int s2 = fp64_residual<float>(gr.nn, gr.rp, gr.cols, A32, x, b, r, k32.partials, &gs->rnorm_out, st))
-          return s2;
+        if (int s2 = matrix32(gr, A32).residual(gr.nn, x, b, r, k32.partials, &gs->rnorm_out, st)) return s2;
         if (seg_out.on()) {
-          if (int s2 = segment_sumsq<double>(seg_out, r, seg_out.r2, st)) return s2;
-          if (int s2 = segment_max_ratio(seg_out, &gs->rel_seg, st)) return s2;
+          if (int s2 = segment_ratio(seg_out, r, &gs->rel_seg, st)) return s2;
         }
         k_ir_next<<<1, 1, 0, st>>>(hir, gs, gb.ctr, ir_body);
         count_launches(1);

@@ -16,6 +16,7 @@ struct ScalarGraph {
   int nn = 0;
   int *rp = nullptr, *cols = nullptr, *diag = nullptr;
   const int *h_rp = nullptr, *h_cols = nullptr, *h_diag = nullptr;
+  EllGraph ell;  // fixed-width storage of the graph, where it has one
 };
 
 // Device state of a graph-captured scalar solve: the refinement loop of the
@@ -97,8 +98,8 @@ struct ScalarSolve {
   // disjoint systems solved as one: a solve converges when every segment
   // does (inner Krylov tests on seg_in, the refinement test on seg_out)
   Segments seg_in, seg_out;
-  int* seg_dev = nullptr;      // [nseg + 1 + nn] row pointers and rows
-  double* seg_buf = nullptr;   // [4 nseg] sums of squares
+  int* seg_dev = nullptr;      // chunk bounds, the segments' chunk ranges, rows, ticket
+  double* seg_buf = nullptr;   // [4 nseg] sums of squares, [nchunk] chunk sums
   double* seg_rel = nullptr;   // device scalar: refinement's largest segment ratio
   int set_segments(const std::vector<int>& ptr, const std::vector<int>& rows);
   void release_segments();
@@ -113,7 +114,14 @@ struct ScalarSolve {
     return 0;
   }
 
-  int init(int n);
+  int init(const ScalarGraph& g, bool mixed);
+  // the solve's matrix in fixed-width storage
+  void* ell = nullptr;
+  size_t ell_size = 0;
+  int widen_matrix(const ScalarGraph& g, bool mixed, const void* A, cudaStream_t st);
+  KrylovMatrix<float> matrix32(const ScalarGraph& g, const float* A) const {
+    return {g.rp, g.cols, A, g.ell, g.ell.w ? static_cast<const float*>(ell) : nullptr};
+  }
   // A: const double* (mixed = false) or const float* (mixed = true); b and x
   // FP64 device vectors of g.nn; x is overwritten. refinements may be null.
   int solve(const ScalarGraph& g, bool mixed, bool amg, bool graphs, const void* A, const double* b, double* x,

@@ -36,9 +36,9 @@
 namespace {
 
 constexpr int kMaxRows = OA_STATIC_SOLVE_MAX_ROWS;
-// 8 Krylov vectors + Jacobi inverse + reduction partials + scalars, with the
-// 256-byte sub-allocation padding KrylovSolver::attach uses
-constexpr size_t kScratchDoubles = 9 * (size_t)kMaxRows + 3 * 2048 + 4096;
+// 8 Krylov vectors + Jacobi inverse + reduction partials (6 x 1,184) + scalars,
+// with the 256-byte sub-allocation padding KrylovSolver::attach uses
+constexpr size_t kScratchDoubles = 9 * (size_t)kMaxRows + 6 * 1184 + 3136;
 
 static __device__ __align__(256) double g_static_scratch[kScratchDoubles];
 
