@@ -27,9 +27,13 @@
 namespace oa {
 
 constexpr int KB = 256;        // threads per block for vector kernels
-// Blocks of the kernels that reduce (8 per SM; they loop over the rows), so
-// that the kernel which uses a sum can add the partials itself, in every block
-constexpr int MAX_PARTIALS = 8 * 148;
+// Blocks of the kernels that reduce; they loop over the rows, so that the
+// kernel which uses a sum can add the partials itself, in every block. The
+// number and the order of the tree below fix the sums' last bits, which
+// BiCGStab in FP32 carries on: with 8 blocks per SM (1184) and the warps added
+// first, twenty momentum iterations ended 1e-7 away in U, and p, whose level
+// hangs on one node, 7e-5.
+constexpr int MAX_PARTIALS = 2048;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -59,11 +63,12 @@ __device__ __forceinline__ void block_partials(double (&v)[NV], double* partials
   }
 }
 
-// ordered sum of nb partials per value, in every thread
+// Sum of nb partials per value in a fixed tree, in every thread: the eight warps
+// first, by halves, then the lanes
 template <int NV>
 __device__ __forceinline__ void sum_partials(const double* __restrict__ partials, int nb, double (&out)[NV]) {
-  __shared__ double sh[NV][KB / 32];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  __shared__ double sh[NV][KB];
+  const int l = threadIdx.x & 31;
   double t[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) t[k] = 0.0;
@@ -71,17 +76,20 @@ __device__ __forceinline__ void sum_partials(const double* __restrict__ partials
 #pragma unroll
     for (int k = 0; k < NV; ++k) t[k] += __ldg(partials + k * MAX_PARTIALS + i);
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const double s = warp_sum(t[k]);
-    if (l == 0) sh[k][w] = s;
-  }
+  for (int k = 0; k < NV; ++k) sh[k][threadIdx.x] = t[k];
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    double s = 0.0;
+    double s[KB / 32];
 #pragma unroll
-    for (int i = 0; i < KB / 32; ++i) s += sh[k][i];
-    out[k] = s;
+    for (int i = 0; i < KB / 32; ++i) s[i] = sh[k][32 * i + l];
+#pragma unroll
+    for (int h = KB / 64; h > 0; h >>= 1)
+#pragma unroll
+      for (int i = 0; i < h; ++i) s[i] += s[i + h];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+    out[k] = s[0];
   }
 }
 
