@@ -115,11 +115,11 @@ struct Flow {
   // production and the previous-iteration k [nn]
   double *mut = nullptr, *F1 = nullptr, *Pk = nullptr, *k_prev = nullptr;
   double urf_k = 1.0, urf_w = 1.0;
-  // [ne][12] Rhie-Chow mass flux of each SCS ip with the pressure-correction
+  // [12][ne] Rhie-Chow mass flux of each SCS ip with the pressure-correction
   // equation's upwind density (its right-hand side), written by the mass-flow
   // kernel and summed per row by the pressure-correction kernel
   double* pc_flux = nullptr;
-  // [ne][8][3] pressure-correction lhs coefficients per element corner (edge
+  // [8][3][ne] pressure-correction lhs coefficients per element corner (edge
   // neighbours in the row-slot order), matrix precision, staged the same way
   void* pc_coef = nullptr;
   // mixed form only: [ne][8] FP32 corner offsets from corner 0 (static) and

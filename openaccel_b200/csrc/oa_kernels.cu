@@ -194,15 +194,16 @@ __device__ __forceinline__ void write_row(int row, bool rv, int li, int lane, co
 // Split in two: the element-owner mass-flow kernel (k_mdot below) evaluates
 // every SCS ip once and stages, per element corner, the lhs coefficients of
 // the corner's three edge neighbours summed over the corner's three ips
-// ([ne][8][3], in the order of edge_nbr) and, per ip, the Rhie-Chow flux of the
-// rhs ([ne][12]); this row kernel gathers its row's eight corner records and
+// ([8][3][ne], in the order of edge_nbr) and, per ip, the Rhie-Chow flux of the
+// rhs ([12][ne]), entry by entry so that a warp of the element kernel stores
+// contiguous values; this row kernel gathers its row's eight corner records and
 // writes the CSR row. The diagonal is minus the sum of the kept neighbour
 // coefficients (partition of unity, sum_n grad N_n = 0: every column outside
 // the edge stencil is lumped into it).
 struct PcArgs {
   MeshView m;
-  const void* coef;    // [ne][8][3] staged lhs coefficients (TF)
-  const double* flux;  // [ne][12] Rhie-Chow ip mass fluxes with the upwind density
+  const void* coef;    // [8][3][ne] staged lhs coefficients (TF)
+  const double* flux;  // [12][ne] Rhie-Chow ip mass fluxes with the upwind density
   void* A;
   double* b;
   const uint8_t* ref_flag;  // [nn] 1 on pressure-level rows
@@ -220,15 +221,15 @@ __global__ void __launch_bounds__(BLOCK) k_pcorr(PcArgs a) {
   TF nb[3][1] = {{TF(0)}, {TF(0)}, {TF(0)}};
   double rhs = 0.0;
   if (e >= 0) {
-    const TF* cf = static_cast<const TF*>(a.coef) + 24 * (size_t)e + 3 * c;
+    const TF* cf = static_cast<const TF*>(a.coef) + (size_t)(3 * c) * a.m.ne + e;
 #pragma unroll
-    for (int s = 0; s < 3; ++s) nb[s][0] = __ldg(cf + s);
+    for (int s = 0; s < 3; ++s) nb[s][0] = __ldg(cf + s * (size_t)a.m.ne);
     diag[0] = -(nb[0][0] + nb[1][0] + nb[2][0]);
     const uint32_t iw = ip_word(c);
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
       const int pk = (iw >> (5 * q)) & 31;
-      const double fl = __ldg(a.flux + 12 * e + (pk >> 1));
+      const double fl = __ldg(a.flux + (size_t)(pk >> 1) * a.m.ne + e);
       rhs -= (pk & 1) ? -fl : fl;
     }
   }
@@ -762,8 +763,8 @@ struct MdotArgs {
   const double *U, *p, *gradP, *du, *rho;
   const double* du_lhs;  // diffusivity of the pressure-correction lhs: D, or D~ with SIMPLEC
   double* mDot;
-  double* flux;  // [ne][12] pressure-correction ip fluxes (staging modes)
-  void* coef;    // [ne][8][3] pressure-correction lhs coefficients per corner (staging modes)
+  double* flux;  // [12][ne] pressure-correction ip fluxes (staging modes)
+  void* coef;    // [8][3][ne] pressure-correction lhs coefficients per corner (staging modes)
   double urf;
   int init;       // initial mass flow rho U.A (no Rhie-Chow term, no fluxes)
   int flux_only;  // write the fluxes from the current mass flow, leave it unchanged
@@ -944,7 +945,7 @@ __global__ void __launch_bounds__(BLOCK, STAGE ? 3 : 4) k_mdot(MdotArgs a) {
           mm += rhoHR * u[j] * Aip[j];
           mm -= rhoHR * duip[j] * (dp[j] - Gp[j]) * Aip[j];
         }
-        a.flux[12 * e + IP] = mm;
+        a.flux[(size_t)IP * a.m.ne + e] = mm;
         // lhs: the flux's dependence on the pressure correction, -rhoHR DU_ip
         // A . grad N_n, for the edge neighbours of L (added to L's row) and of
         // R (subtracted from R's row: the ip's area points away from L)
@@ -968,11 +969,11 @@ __global__ void __launch_bounds__(BLOCK, STAGE ? 3 : 4) k_mdot(MdotArgs a) {
     }
   });
   if constexpr (STAGE) {
-    TC* out = static_cast<TC*>(a.coef) + 24 * (size_t)e;
+    TC* out = static_cast<TC*>(a.coef) + e;
 #pragma unroll
     for (int k = 0; k < 8; ++k)
 #pragma unroll
-      for (int sl = 0; sl < 3; ++sl) out[3 * k + sl] = coef[k][sl];
+      for (int sl = 0; sl < 3; ++sl) out[(3 * k + sl) * (size_t)a.m.ne] = coef[k][sl];
   }
   if (err) a.err[0] = 1;
 }
