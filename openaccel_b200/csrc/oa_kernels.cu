@@ -401,9 +401,11 @@ __device__ __forceinline__ void sym_face(const TF (&x)[8][3], const TF (&Uc)[8][
 // geometry (upwind advection with the same mass flows, diffusion with the
 // nodal diffusivities at the ips: phiAssemblerElemTerms.hpp:11-413, N = 1);
 // VAR 0 is the steady upwind SIMPLE assembly with nothing else in its
-// register budget.
+// register budget. Blocks per SM, measured at 128^3: FP32 4 (1,781 us; 3: 2,192,
+// 5 spills: 1,858), FP64 3 (3,243 us in 168 registers with a few spills; 2:
+// 3,626, 4: 4,106).
 template <int LPR, bool USH, bool UGSH, class TF, int VAR = 0>
-__global__ void __launch_bounds__(BLOCK, sizeof(TF) == 4 ? (UGSH ? 4 : 3) : 1)
+__global__ void __launch_bounds__(BLOCK, sizeof(TF) == 4 ? (UGSH ? 4 : 3) : (UGSH ? 3 : 1))
     k_momentum(MomArgs a) {
   constexpr bool EXT = VAR == 1;
   constexpr bool TURB = VAR == 2;
