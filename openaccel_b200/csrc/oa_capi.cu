@@ -433,9 +433,7 @@ int build_iteration_graph(oa_flow* h) {
         count_launches(1);
         if (int s2 = launch_update_mdot(f)) return s2;
         if (int s2 = launch_div(f)) return s2;
-        if (int s2 = launch_axpy_du_gradp(f, +1.0)) return s2;
-        if (int s2 = launch_gradient(f, 0)) return s2;
-        if (int s2 = launch_axpy_du_gradp(f, -1.0)) return s2;
+        if (int s2 = launch_correct_velocity(f)) return s2;
         if (int s2 = launch_gradient(f, 1)) return s2;
         if (f.s.hr)
           if (int s2 = launch_blend_u(f)) return s2;
@@ -827,6 +825,11 @@ int oa_flow_create(oa_mesh* M, const oa_flow_settings* s, const double* bnd_velo
       return st;
     }
   }
+  // block meshes: at most six edges at a node
+  if (s->precision == OA_PREC_FP64 && M->m.lpr == 8 && M->m.ell.w == 7 && (st = launch_edge_areas(f))) {
+    oa_flow_destroy(H);
+    return st;
+  }
   // constant properties, zero fields
   std::vector<double> h(nn, s->rho);
   cudaMemcpy(f.rho, h.data(), sizeof(double) * nn, cudaMemcpyHostToDevice);
@@ -888,7 +891,8 @@ void oa_flow_destroy(oa_flow* H) {
                   f.betaU,   f.minU,    f.maxU,    f.duT,     f.Uold,    f.Uoldold, f.kf,      f.wf,
                   f.gkf,     f.gwf,     f.sdk,     f.srk,     f.sdw,     f.srw,     f.A_k,     f.b_k,
                   f.A_w,     f.b_w,     f.sym_mask, f.sym_nodes, f.sym_area, f.wall_face_node,
-                  f.gradK,   f.gradW,   f.mut,     f.F1,      f.Pk,      f.k_prev};
+                  f.gradK,   f.gradW,   f.mut,     f.F1,      f.Pk,      f.k_prev,
+                  f.edge_node, f.edge_area};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (H->hscal) cudaFreeHost(H->hscal);
@@ -1214,9 +1218,8 @@ int oa_simple_iterate(oa_flow* H, int n, oa_iter_stats* stats) {
     if (!s) {
       k_axpy<<<(f.mesh->nn + 255) / 256, 256, 0, f.stream>>>(f.mesh->nn, f.p, f.b.x_pc, f.s.urf_p);
       count_launches(1);
-      if (!(s = launch_update_mdot(f)) && !(s = launch_div(f)) && !(s = launch_axpy_du_gradp(f, +1.0)) &&
-          !(s = launch_gradient(f, 0)) && !(s = launch_axpy_du_gradp(f, -1.0)) && !(s = launch_gradient(f, 1)) &&
-          f.s.hr)
+      if (!(s = launch_update_mdot(f)) && !(s = launch_div(f)) && !(s = launch_correct_velocity(f)) &&
+          !(s = launch_gradient(f, 1)) && f.s.hr)
         s = launch_blend_u(f);  // segregatedFlowEquations.cpp:287-288
     }
     nvtxRangePop();

@@ -122,6 +122,12 @@ struct Flow {
   // [8][3][ne] pressure-correction lhs coefficients per element corner (edge
   // neighbours in the row-slot order), matrix precision, staged the same way
   void* pc_coef = nullptr;
+  // FP64 on block meshes: the up to six edge neighbours of each node and the SCS
+  // area vectors of the edges, summed over the elements around each and
+  // pointing away from the node, in groups of 32 nodes: [nn/32][6][32] and
+  // [nn/32][6][3][32] (null: none)
+  int* edge_node = nullptr;
+  double* edge_area = nullptr;
   // mixed form only: [ne][8] FP32 corner offsets from corner 0 (static) and
   // the [nn] FP32 (U, mu) copy packed before each momentum assembly
   float4* xloc32 = nullptr;
@@ -195,11 +201,14 @@ int launch_pcorr(Flow& f, bool mixed, bool flux_fresh = false);
 int launch_momentum(Flow& f, bool mixed);
 int launch_init_mdot(Flow& f);
 int launch_xloc(Flow& f);
+int launch_edge_areas(Flow& f);
 // stage: also write the pressure-correction ip fluxes and corner coefficients
 int launch_update_mdot(Flow& f, bool stage = false);
 int launch_div(Flow& f);
 int launch_gradient(Flow& f, int which);
-int launch_axpy_du_gradp(Flow& f, double sign);
+// the pressure gradient after a correction and, around it, the velocity
+// correction: U += D grad p / urf_p, grad p updated, U -= D grad p / urf_p
+int launch_correct_velocity(Flow& f);
 // velocity extrema and blending factor of the high-resolution scheme
 int launch_blend_u(Flow& f);
 // assembled symmetry area [nn][3] of every node (zero off the symmetry planes)
