@@ -35,6 +35,8 @@ constexpr int KB = 256;        // threads per block for vector kernels
 // hangs on one node, 7e-5.
 constexpr int MAX_PARTIALS = 2048;
 
+// of a solver: two sets of two values
+constexpr int KRYLOV_PARTIALS = 4 * MAX_PARTIALS;
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -563,7 +565,7 @@ int KrylovSolver<B, TM, TV>::setup(int nn_, const int* rp_, const int* cols_, co
   const size_t n = (size_t)B * nn;
   for (int k = 0; k < 8; ++k) OA_CUDA(cudaMalloc(&vec[k], sizeof(TV) * n));
   OA_CUDA(cudaMalloc(&Minv, sizeof(double) * (size_t)B * B * nn));
-  OA_CUDA(cudaMalloc(&partials, sizeof(double) * partials_size()));
+  OA_CUDA(cudaMalloc(&partials, sizeof(double) * KRYLOV_PARTIALS));
   OA_CUDA(cudaMalloc(&scal, sizeof(KScal)));
   OA_CUDA(cudaMallocHost(&hscal, sizeof(KScal)));
   return OA_OK;
@@ -573,7 +575,7 @@ template <int B, class TM, class TV>
 size_t KrylovSolver<B, TM, TV>::storage_bytes(int nn_) {
   const size_t n = (size_t)B * nn_;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  return 8 * up(sizeof(TV) * n) + up(sizeof(double) * (size_t)B * B * nn_) + up(sizeof(double) * partials_size()) +
+  return 8 * up(sizeof(TV) * n) + up(sizeof(double) * (size_t)B * B * nn_) + up(sizeof(double) * KRYLOV_PARTIALS) +
          up(sizeof(KScal));
 }
 
@@ -598,7 +600,7 @@ int KrylovSolver<B, TM, TV>::attach(int nn_, const int* rp_, const int* cols_, c
   Minv = reinterpret_cast<double*>(p);
   p += up(sizeof(double) * (size_t)B * B * nn);
   partials = reinterpret_cast<double*>(p);
-  p += up(sizeof(double) * partials_size());
+  p += up(sizeof(double) * KRYLOV_PARTIALS);
   scal = p;
   return OA_OK;
 }

@@ -36,9 +36,9 @@
 namespace {
 
 constexpr int kMaxRows = OA_STATIC_SOLVE_MAX_ROWS;
-// 8 Krylov vectors + Jacobi inverse + reduction partials (6 x 1,184) + scalars,
+// 8 Krylov vectors + Jacobi inverse + reduction partials (4 x 2,048) + scalars,
 // with the 256-byte sub-allocation padding KrylovSolver::attach uses
-constexpr size_t kScratchDoubles = 9 * (size_t)kMaxRows + 6 * 1184 + 3136;
+constexpr size_t kScratchDoubles = 9 * (size_t)kMaxRows + 4 * 2048 + 2048;
 
 static __device__ __align__(256) double g_static_scratch[kScratchDoubles];
 
