@@ -303,13 +303,12 @@ struct RowMat {
   int n;
   const int *rp, *cols;
   const T* A;
-  const int* ecols;
-  const T* eval;
+  EllMat<T> ell;
 };
 
 template <int LPR, class T, class G>
 __device__ __forceinline__ double mat_row(const RowMat<T>& m, int i, int lane, G get) {
-  if constexpr (LPR >= ELL) return i < m.n ? ell_row<LPR, T>(m.ecols, m.eval, i, get) : 0.0;
+  if constexpr (LPR >= ELL) return i < m.n ? ell_row<LPR, T>(m.ell, i, get) : 0.0;
   int a = 0, e = 0;
   if (i < m.n) {
     a = __ldg(m.rp + i);
@@ -776,7 +775,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1)
 // ---------------------------------------------------------------------------
 template <class T>
 static RowMat<T> level_matrix(const AmgLevel<T>& v) {
-  return {v.n, v.rp, v.cols, v.A, v.ell.cols, v.ell_val};
+  return {v.n, v.rp, v.cols, v.A, ell_mat(v.ell, v.ell_val)};
 }
 template <class T>
 static int level_format(const AmgLevel<T>& v) {

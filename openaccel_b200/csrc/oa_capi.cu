@@ -735,7 +735,7 @@ void oa_mesh_destroy(oa_mesh* M) {
   DeviceMesh& m = M->m;
   void* ptrs[] = {m.x,       m.conn,      m.n2e,      m.n2e_ptr,  m.n2f,       m.n2f_ptr, m.face_elem, m.face_ord,
                   m.face_bnd, m.row_ptr, m.cols,     m.diag,     m.face_mask, m.vol,     m.wscv,      m.wall_node,
-                  m.scs_area, m.slot_mask, m.slot_mask64, const_cast<int*>(m.ell.cols)};
+                  m.scs_area, m.slot_mask, m.slot_mask64, m.ell.cols};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (M->st) cudaStreamDestroy(M->st);

@@ -1,19 +1,29 @@
 // Fixed-width row storage of a scalar CSR matrix (internal).
 //
-// Rows come in groups of 32; entry q of row i sits at 32 (W (i / 32) + q) + i % 32.
+// Rows come in groups of 32; slot q of row i sits at 32 (W (i / 32) + q) + i % 32.
 // A warp whose lanes take one row each then reads every slot as one contiguous
-// line of values and one of columns (in CSR the same loads are strided by the
-// row length), needs no row pointer in its chain of dependent loads, and has
-// all W slots in flight at once. W is a compile-time constant, for the two row
-// lengths of the stencils this library assembles: 7 (a node of a hex block and
-// its edge neighbours) and 15 (a node of a block split into Kuhn tets). Other
-// graphs keep CSR, and so does one that the padding would more than double.
-// Measured product, matrix in DRAM: 97^3 rows FP64 14.8 us (CSR 22.8), 129^3 rows
-// FP32 20.7 us (CSR 32.8), that is 6.2 and 6.6 TB/s; a run-time width lost most
-// of it (20.7 and 28.9 us). Entries past a row's end have value 0 and the row's
-// first column (0 in an empty row).
+// line of values (in CSR the same loads are strided by the row length), needs no
+// row pointer in its chain of dependent loads, and has all W slots in flight at
+// once. W is a compile-time constant, for the two row lengths of the stencils
+// this library assembles: 7 (a node of a hex block and its edge neighbours) and
+// 15 (a node of a block split into Kuhn tets). Other graphs keep CSR, and so
+// does one that the padding would more than double.
+//
+// In a block's numbering the 32 rows of a group have their columns at the same
+// few distances, so a group keeps the distances once where W of them hold all its
+// rows' columns, and a row the set of slots it has (2 bytes): the product is
+// bound by DRAM, and columns of 4 bytes per entry are half of an FP32 matrix.
+// Groups with more distances (ends of blocks, unordered meshes) read columns.
+//
+// Measured product, matrix in DRAM: 97^3 rows FP64 CSR 22.8 us, with columns 14.8;
+// 129^3 rows FP32 32.8 and 20.7; a run-time width lost most of it (20.7 and 28.9
+// us). On 129^3 rows FP32 with columns and with distances: smoothing step with
+// residual 24.7 and 22.8 us, smoothing step 23.8 and 20.9, product in GCR 26.6
+// and 24.7. Absent slots have value 0 and a column of the row itself.
 #pragma once
 #include <cuda_runtime.h>
+
+#include <cstdint>
 
 namespace oa {
 
@@ -24,15 +34,31 @@ namespace oa {
 constexpr int ELL = 100, ELL_STREAM = 200;
 constexpr long long ELL_STREAM_BYTES = 32 << 20;
 
+// Width that keeps distances; with 15 of them the products ran out of registers
+// (conduction on 65^3 nodes, mixed: 2.47 ms with columns, 2.90 with distances).
+constexpr int ELL_DISTANCES = 7;
+
 constexpr int lanes_of(int format) { return format >= ELL ? 1 : format; }
 
 struct EllGraph {
   int w = 0;  // 0: the graph has none
-  const int* cols = nullptr;
+  int* cols = nullptr;  // [n/32][W][32], and after it in the same allocation:
+  const int* delta = nullptr;       // [n/32][W + 1] distances; 1 last where the rows read columns
+  const uint16_t* mask = nullptr;   // [n] slots of each row
   long long slots = 0;
 };
+template <class T>
+struct EllMat {
+  const int *cols, *delta;
+  const uint16_t* mask;
+  const T* val;
+};
+template <class T>
+inline EllMat<T> ell_mat(const EllGraph& g, const T* val) {
+  return {g.cols, g.delta, g.mask, val};
+}
 inline int ell_format(int w, long long slots, size_t value_bytes) {
-  return w ? (slots * (long long)(value_bytes + sizeof(int)) > ELL_STREAM_BYTES ? ELL_STREAM : ELL) + w : 1;
+  return w ? (slots * (long long)value_bytes > ELL_STREAM_BYTES ? ELL_STREAM : ELL) + w : 1;
 }
 
 template <bool STREAM, class X>
@@ -42,16 +68,35 @@ __device__ __forceinline__ X ell_load(const X* p) {
 
 // sum of value * get(column) over row i, in slot order
 template <int FORMAT, class T, class G>
-__device__ __forceinline__ double ell_row(const int* __restrict__ cols, const T* __restrict__ val, int i, G get) {
+__device__ __forceinline__ double ell_row(const EllMat<T>& m, int i, G get) {
   constexpr int W = FORMAT % 100;
   constexpr bool STREAM = FORMAT >= ELL_STREAM;
   const size_t at = (size_t)(i >> 5) * (32 * W) + (i & 31);
-  int j[W];
   T v[W];
+  int j[W + 1];
 #pragma unroll
-  for (int q = 0; q < W; ++q) {
-    j[q] = ell_load<STREAM>(cols + at + 32 * q);
-    v[q] = ell_load<STREAM>(val + at + 32 * q);
+  for (int q = 0; q < W; ++q) v[q] = ell_load<STREAM>(m.val + at + 32 * q);
+  if constexpr (W == ELL_DISTANCES) {
+    const unsigned mask = __ldg(m.mask + i);
+    const int4* d = reinterpret_cast<const int4*>(m.delta + (size_t)(i >> 5) * (W + 1));
+#pragma unroll
+    for (int q = 0; q < W + 1; q += 4) {
+      const int4 t = __ldg(d + q / 4);
+      j[q] = t.x;
+      j[q + 1] = t.y;
+      j[q + 2] = t.z;
+      j[q + 3] = t.w;
+    }
+    if (j[W]) {
+#pragma unroll
+      for (int q = 0; q < W; ++q) j[q] = ell_load<STREAM>(m.cols + at + 32 * q);
+    } else {
+#pragma unroll
+      for (int q = 0; q < W; ++q) j[q] = mask >> q & 1 ? i + j[q] : i;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < W; ++q) j[q] = ell_load<STREAM>(m.cols + at + 32 * q);
   }
   double s = 0.0;
 #pragma unroll
@@ -59,11 +104,10 @@ __device__ __forceinline__ double ell_row(const int* __restrict__ cols, const T*
   return s;
 }
 
-// Width and device columns of a graph (w 0 where it keeps CSR); the caller frees
-// the columns.
+// Width and device graph (w 0 where it keeps CSR); the caller frees cols.
 int ell_graph(int n, const int* h_rp, const int* rp, const int* cols, EllGraph* out, cudaStream_t st);
-// values of a CSR matrix into the fixed-width storage (padding zero)
+// values of a CSR matrix into the fixed-width storage (absent slots zero)
 template <class T>
-int ell_values(int n, const int* rp, const T* csr, int w, T* out, cudaStream_t st);
+int ell_values(int n, const int* rp, const T* csr, const EllGraph& g, T* out, cudaStream_t st);
 
 }  // namespace oa

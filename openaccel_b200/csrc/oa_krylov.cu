@@ -16,6 +16,7 @@
 #include <cstdlib>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <vector>
 #include <type_traits>
@@ -34,9 +35,9 @@ constexpr int KB = 256;        // threads per block for vector kernels
 // first, twenty momentum iterations ended 1e-7 away in U, and p, whose level
 // hangs on one node, 7e-5.
 constexpr int MAX_PARTIALS = 2048;
-
 // of a solver: two sets of two values
 constexpr int KRYLOV_PARTIALS = 4 * MAX_PARTIALS;
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -265,13 +266,12 @@ template <class TM>
 struct ScalarMat {
   const int *rp, *cols;  // CSR
   const TM* A;
-  const int* ecols;      // fixed-width storage
-  const TM* eval;
+  EllMat<TM> ell;        // fixed-width storage
 };
 template <int FORMAT, class TM, class TX>
 __device__ __forceinline__ double scalar_row(const ScalarMat<TM>& m, int i, const TX* __restrict__ x) {
   if constexpr (FORMAT >= ELL)
-    return ell_row<FORMAT, TM>(m.ecols, m.eval, i, [&](int j) { return double(__ldg(x + j)); });
+    return ell_row<FORMAT, TM>(m.ell, i, [&](int j) { return double(__ldg(x + j)); });
   else
     return row_product<1, TM, TX>(m.cols, m.A, x, __ldg(m.rp + i), __ldg(m.rp + i + 1), 0);
 }
@@ -678,7 +678,7 @@ int KrylovSolver<B, TM, TV>::chunk(const TM* A, int check_every, bool use_gcr) {
   const int gv = reduce_grid(n);
   // two sets of partials: a kernel reads the one and writes the other
   double *pa = partials, *pb = partials + 2 * MAX_PARTIALS;
-  const ScalarMat<TM> M = {rp, cols, A, ell.cols, static_cast<const TM*>(ell_val)};
+  const ScalarMat<TM> M = {rp, cols, A, ell_mat(ell, static_cast<const TM*>(ell_val))};
   const int format = B == 1 && ell_val ? ell_format(ell.w, ell.slots, sizeof(TM)) : 1;
   if (use_gcr) {
     // GCR(2) work vectors in the same buffers: x r z q P0 P1 Q0 Q1
@@ -851,22 +851,42 @@ OA_EMIT(3, float, float, float)
 
 // ---------------------------------------------------------------------------
 // fixed-width storage
-__global__ void k_ell_cols(int n, int w, const int* rp, const int* cols, int* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (n + 31) / 32 * 32) return;
-  const int a = i < n ? rp[i] : 0, len = i < n ? rp[i + 1] - a : 0, pad = len ? cols[a] : 0;
-  for (int q = 0; q < w; ++q) out[(size_t)(i >> 5) * 32 * w + 32 * q + (i & 31)] = q < len ? cols[a + q] : pad;
+// One warp per group. Its distances are merged from the rows' column lists, the
+// smallest next one first, so that every row keeps its order.
+__global__ void __launch_bounds__(32) k_ell_graph(int n, int w, const int* rp, const int* cols, int* out, int* delta,
+                                                  uint16_t* mask) {
+  const int i = blockIdx.x * 32 + threadIdx.x;
+  const int a = i < n ? rp[i] : 0, len = i < n ? rp[i + 1] - a : 0;
+  int* d = delta + (size_t)blockIdx.x * (w + 1);
+  int at = 0;
+  unsigned have = 0;
+  for (int q = 0; q < w; ++q) {
+    const int next = at < len ? cols[a + at] - i : INT_MAX;
+    const int m = __reduce_min_sync(0xffffffffu, next);
+    if (next == m && m != INT_MAX) {
+      have |= 1u << q;
+      ++at;
+    }
+    if (threadIdx.x == 0) d[q] = m == INT_MAX ? 0 : m;
+  }
+  const bool columns = w != ELL_DISTANCES || __any_sync(0xffffffffu, at < len);
+  const int pad = len ? cols[a] : 0;
+  if (threadIdx.x == 0) d[w] = columns;
+  mask[i] = (uint16_t)(columns ? (1u << len) - 1 : have);
+  for (int q = 0; q < w; ++q) out[(size_t)blockIdx.x * 32 * w + 32 * q + threadIdx.x] = q < len ? cols[a + q] : pad;
 }
 
 template <class T, int W>
-__global__ void __launch_bounds__(256) k_ell_values(int n, const int* __restrict__ rp, const T* __restrict__ csr,
+__global__ void __launch_bounds__(256) k_ell_values(int n, const int* __restrict__ rp,
+                                                    const uint16_t* __restrict__ mask, const T* __restrict__ csr,
                                                     T* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (n + 31) / 32 * 32) return;
-  const int a = i < n ? __ldg(rp + i) : 0, len = i < n ? __ldg(rp + i + 1) - a : 0;
+  const int a = i < n ? __ldg(rp + i) : 0;
+  const unsigned have = __ldg(mask + i);
   T v[W];
 #pragma unroll
-  for (int q = 0; q < W; ++q) v[q] = q < len ? __ldg(csr + a + q) : T(0);
+  for (int q = 0; q < W; ++q) v[q] = have >> q & 1 ? __ldg(csr + a + __popc(have & ((1u << q) - 1))) : T(0);
 #pragma unroll
   for (int q = 0; q < W; ++q) out[(size_t)(i >> 5) * 32 * W + 32 * q + (i & 31)] = v[q];
 }
@@ -876,31 +896,36 @@ int ell_graph(int n, const int* h_rp, const int* rp, const int* cols, EllGraph* 
   int longest = 0;
   for (int i = 0; i < n; ++i) longest = std::max(longest, h_rp[i + 1] - h_rp[i]);
   const int w = longest <= 7 ? 7 : 15;
-  const long long slots = (n + 31LL) / 32 * 32 * w;
+  const long long groups = (n + 31LL) / 32, slots = groups * 32 * w;
   if (longest > w || slots > 2LL * h_rp[n] + 4096) return OA_OK;
   int* c = nullptr;
-  if (cudaMalloc(&c, sizeof(int) * slots) != cudaSuccess)
+  if (cudaMalloc(&c, sizeof(int) * (slots + groups * (w + 1)) + sizeof(uint16_t) * groups * 32) != cudaSuccess)
     return fail(OA_ERR_CUDA, "fixed-width matrix storage: allocation failed");
+  int* delta = c + slots;
+  uint16_t* mask = reinterpret_cast<uint16_t*>(delta + groups * (w + 1));
   out->w = w;
   out->cols = c;
+  out->delta = delta;
+  out->mask = mask;
   out->slots = slots;
-  k_ell_cols<<<(n + 31) / 32 * 32 / 32, 32, 0, st>>>(n, w, rp, cols, c);
+  if (groups == 0) return OA_OK;
+  k_ell_graph<<<(unsigned)groups, 32, 0, st>>>(n, w, rp, cols, c, delta, mask);
   count_launches(1);
   OA_CUDA(cudaGetLastError());
   return OA_OK;
 }
 
 template <class T>
-int ell_values(int n, const int* rp, const T* csr, int w, T* out, cudaStream_t st) {
+int ell_values(int n, const int* rp, const T* csr, const EllGraph& gr, T* out, cudaStream_t st) {
   const int g = ((n + 31) / 32 * 32 + 255) / 256;
-  if (w == 7) k_ell_values<T, 7><<<g, 256, 0, st>>>(n, rp, csr, out);
-  else k_ell_values<T, 15><<<g, 256, 0, st>>>(n, rp, csr, out);
+  if (gr.w == 7) k_ell_values<T, 7><<<g, 256, 0, st>>>(n, rp, gr.mask, csr, out);
+  else k_ell_values<T, 15><<<g, 256, 0, st>>>(n, rp, gr.mask, csr, out);
   count_launches(1);
   OA_CUDA(cudaGetLastError());
   return OA_OK;
 }
-template int ell_values<float>(int, const int*, const float*, int, float*, cudaStream_t);
-template int ell_values<double>(int, const int*, const double*, int, double*, cudaStream_t);
+template int ell_values<float>(int, const int*, const float*, const EllGraph&, float*, cudaStream_t);
+template int ell_values<double>(int, const int*, const double*, const EllGraph&, double*, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // FP64 residual for iterative refinement: r = b - A x (A in its stored
@@ -938,7 +963,7 @@ template <class TM>
 int KrylovMatrix<TM>::residual(int nn, const double* x, const double* b, double* r, double* partials,
                                double* norm_dev, cudaStream_t st) const {
   const int g = reduce_grid(nn);
-  const ScalarMat<TM> M = {rp, cols, A, ell.cols, eval};
+  const ScalarMat<TM> M = {rp, cols, A, ell_mat(ell, eval)};
 #define OA_CALL(F) k_residual<TM, F><<<g, KB, 0, st>>>(nn, M, x, b, r, partials)
   OA_FORMAT(eval ? ell_format(ell.w, ell.slots, sizeof(TM)) : 1, OA_CALL)
 #undef OA_CALL

@@ -191,8 +191,8 @@ int ScalarSolve::widen_matrix(const ScalarGraph& g, bool mixed, const void* A, c
   amg64.set_finest(g.ell, static_cast<const double*>(k64.ell_val));
   amg32.set_finest(g.ell, static_cast<const float*>(k32.ell_val));
   if (!on) return OA_OK;
-  return mixed ? ell_values<float>(g.nn, g.rp, static_cast<const float*>(A), g.ell.w, static_cast<float*>(ell), st)
-               : ell_values<double>(g.nn, g.rp, static_cast<const double*>(A), g.ell.w, static_cast<double*>(ell), st);
+  return mixed ? ell_values<float>(g.nn, g.rp, static_cast<const float*>(A), g.ell, static_cast<float*>(ell), st)
+               : ell_values<double>(g.nn, g.rp, static_cast<const double*>(A), g.ell, static_cast<double*>(ell), st);
 }
 
 int ScalarSolve::set_segments(const std::vector<int>& ptr, const std::vector<int>& rows) {
