@@ -96,6 +96,13 @@ __device__ __forceinline__ void sum_partials(const double* __restrict__ partials
   }
 }
 
+// The done flag for a kernel whose first block may set it (a breakdown) while
+// other blocks of the same grid start: one answer for the whole block. With a
+// test by each thread a block could lose some warps to the flag, and the others
+// would add the sums those never wrote and go on with a wrong coefficient. A
+// block that still sees the flag clear finds the same breakdown in the sums.
+__device__ __forceinline__ bool block_done(const KScal* sc) { return __syncthreads_or(sc->done); }
+
 static int reduce_grid(long long n) { return (int)std::min<long long>((n + KB - 1) / KB, MAX_PARTIALS); }
 
 // Product of row component m of block row [a, e) with x: U entries at a time
@@ -235,7 +242,7 @@ template <int B, class TV>
 __global__ void __launch_bounds__(KB) k_s_update(int nn, TV* r, const TV* __restrict__ v,
                                                   const TV* __restrict__ Minv, TV* sh,
                                                   const double* __restrict__ partials, int nb, KScal* sc) {
-  if (sc->done) return;
+  if (block_done(sc)) return;
   double o[1];
   sum_partials<1>(partials, nb, o);
   const bool broken = o[0] == 0.0 || !(fabs(o[0]) < INFINITY);
@@ -527,7 +534,7 @@ __global__ void __launch_bounds__(KB) k_gcr_update(int n, TV* x, TV* r, const TV
                                                     const TV* __restrict__ q, TV* __restrict__ P, TV* __restrict__ Q,
                                                     const double* __restrict__ in, int nb, double* partials,
                                                     KScal* sc) {
-  if (sc->done) return;
+  if (block_done(sc)) return;
   double o[2];
   sum_partials<2>(in, nb, o);
   const double nq = sqrt(o[0]);
