@@ -89,7 +89,6 @@ void Amg<T>::release() {
   L.clear();
   if (dense_inv) cudaFree(dense_inv);
   if (dense_op) cudaFree(dense_op);
-  if (dense_work) cudaFree(dense_work);
   dense_inv = nullptr;
   dense_op = nullptr;
   dense_work = nullptr;
@@ -539,15 +538,15 @@ __global__ void __launch_bounds__(AB) k_up(RowMat<T> m, const T* dinv, const int
   ph_up<T>(m, dinv, agg, b, xs, xc, x, w, alpha);
 }
 
-// x = M b with the dense operator of a level, one warp per row
+// x = M b with the dense operator of a level (rows ld apart), one warp per row
 template <class T>
-__global__ void __launch_bounds__(AB) k_dense_apply(int n, const double* __restrict__ M, const T* __restrict__ b,
-                                                    T* __restrict__ x, const int* done) {
+__global__ void __launch_bounds__(AB) k_dense_apply(int n, const double* __restrict__ M, int ld,
+                                                    const T* __restrict__ b, T* __restrict__ x, const int* done) {
   if (*done) return;
   for_rows<32>(n, [&](int i, int lane) {
     double s = 0.0;
     if (i < n) {
-      const double* row = M + (size_t)i * n;
+      const double* row = M + (size_t)i * ld;
 #pragma unroll 4
       for (int j = lane; j < n; j += 32) s += __ldg(row + j) * double(__ldg(b + j));
     }
@@ -931,13 +930,16 @@ int Amg<T>::setup(int n, const int* h_rp, const int* h_cols, const int* h_diag, 
   // (the finest matrix is always the current one, and an FP32 cycle rounds its
   // vectors after every phase, which the operator would not)
   while (smoothed && sizeof(T) == 8 && tail > 1 && L[tail - 1].n <= DENSE_ROWS) --tail;
-  const size_t nt = L[tail].n;
-  int s;
-  if ((s = dalloc(&dense_op, nt * nt))) return s;
-  if (tail < (int)L.size() - 1) {
+  const int last = (int)L.size() - 1;
+  if (tail < last) {
+    const size_t nt = L[tail].n;
     size_t rows = 0;
     for (size_t l = tail; l < L.size(); ++l) rows += L[l].n;
-    if ((s = dalloc(&dense_work, 6 * rows * std::min<size_t>(nt, DENSE_COLS)))) return s;
+    // operator, then workspace; without room for them the cycle runs through these levels
+    dense_op = static_cast<double*>(
+        spare_alloc(sizeof(double) * (nt * nt + 6 * rows * std::min<size_t>(nt, DENSE_COLS)), n));
+    if (dense_op) dense_work = dense_op + nt * nt;
+    else tail = last;
   }
   ready = true;
   return OA_OK;
@@ -1106,26 +1108,16 @@ __global__ void __launch_bounds__(128) k_inverse_columns(int n, int C, const dou
   x[(size_t)i * C + c] = s;
 }
 
-// columns c0 .. c0 + C into the row-major operator; the coarsest level's
-// operator is its inverse itself
+// columns c0 .. c0 + C into the row-major operator
 __global__ void k_store_columns(int n, int C, int c0, const double* __restrict__ x, double* __restrict__ M) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n * C) M[(size_t)(t / C) * n + c0 + t % C] = x[t];
-}
-__global__ void k_store_inverse(int n, const double* __restrict__ inv, double* __restrict__ M) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n * n) M[t] = inv[(size_t)(t / n) * 2 * n + n + t % n];
 }
 
 template <class T>
 int Amg<T>::dense_operator(cudaStream_t st) {
   const int nl = (int)L.size(), n = L[tail].n;
-  if (tail == nl - 1) {
-    k_store_inverse<<<(n * n + AB - 1) / AB, AB, 0, st>>>(n, dense_inv, dense_op);
-    count_launches(1);
-    OA_CUDA(cudaGetLastError());
-    return OA_OK;
-  }
+  if (tail == nl - 1) return OA_OK;  // the coarsest level's inverse itself
   const int cols = std::min(n, DENSE_COLS);
   struct Cols {
     double *b, *x, *r, *d0, *d1, *t;
@@ -1217,7 +1209,9 @@ int Amg<T>::apply(const T* v, T* z, const int* done, cudaStream_t st) {
   }
   {
     AmgLevel<T>& lv = L[tail];
-    k_dense_apply<T><<<grid_for(lv.n, 32), AB, 0, st>>>(lv.n, dense_op, tail == 0 ? v : lv.b, tail == 0 ? z : lv.x, done);
+    const double* M = dense_op ? dense_op : dense_inv + lv.n;
+    k_dense_apply<T><<<grid_for(lv.n, 32), AB, 0, st>>>(lv.n, M, dense_op ? lv.n : 2 * lv.n, tail == 0 ? v : lv.b,
+                                                        tail == 0 ? z : lv.x, done);
     count_launches(1);
   }
   // upward pass above the dense operator: prolongation + post-smooth (one fused kernel

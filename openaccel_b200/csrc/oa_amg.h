@@ -86,7 +86,8 @@ struct Amg {
   int cheb_rows = 50000;
   double cheb_ratio = 30.0;
   // the cycle from level `tail` down is one dense operator [n][n] (row-major),
-  // formed by the numeric phase in dense_work
+  // formed by the numeric phase in dense_work (both in one allocation); null
+  // where tail is the coarsest level, whose operator is its inverse itself
   int tail = 0;
   double* dense_op = nullptr;
   double* dense_work = nullptr;

@@ -892,7 +892,7 @@ void oa_flow_destroy(oa_flow* H) {
                   f.gkf,     f.gwf,     f.sdk,     f.srk,     f.sdw,     f.srw,     f.A_k,     f.b_k,
                   f.A_w,     f.b_w,     f.sym_mask, f.sym_nodes, f.sym_area, f.wall_face_node,
                   f.gradK,   f.gradW,   f.mut,     f.F1,      f.Pk,      f.k_prev,
-                  f.edge_node, f.edge_area};
+                  f.edge_area};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (H->hscal) cudaFreeHost(H->hscal);

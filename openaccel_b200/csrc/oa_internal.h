@@ -125,7 +125,7 @@ struct Flow {
   // FP64 on block meshes: the up to six edge neighbours of each node and the SCS
   // area vectors of the edges, summed over the elements around each and
   // pointing away from the node, in groups of 32 nodes: [nn/32][6][32] and
-  // [nn/32][6][3][32] (null: none)
+  // [nn/32][6][3][32], in one allocation (null: none)
   int* edge_node = nullptr;
   double* edge_area = nullptr;
   // mixed form only: [ne][8] FP32 corner offsets from corner 0 (static) and
@@ -202,6 +202,9 @@ int launch_momentum(Flow& f, bool mixed);
 int launch_init_mdot(Flow& f);
 int launch_xloc(Flow& f);
 int launch_edge_areas(Flow& f);
+// Device storage for a system of the given rows that makes calls faster but
+// that they can do without: null where it would leave too little for the rest
+void* spare_alloc(size_t bytes, long long rows);
 // stage: also write the pressure-correction ip fluxes and corner coefficients
 int launch_update_mdot(Flow& f, bool stage = false);
 int launch_div(Flow& f);

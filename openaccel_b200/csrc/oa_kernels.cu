@@ -891,15 +891,11 @@ __global__ void __launch_bounds__(BLOCK) k_edge_areas(MeshView m, int* edge_node
 int launch_edge_areas(Flow& f) {
   const DeviceMesh& m = *f.mesh;
   const size_t ng = (m.nn + 31) / 32;
-  if (cudaMalloc(&f.edge_node, sizeof(int) * 192 * ng) != cudaSuccess ||
-      cudaMalloc(&f.edge_area, sizeof(double) * 576 * ng) != cudaSuccess) {
-    // no room (168 B per node): the gradients keep the ip form
-    if (f.edge_node) cudaFree(f.edge_node);
-    f.edge_node = nullptr;
-    f.edge_area = nullptr;
-    cudaGetLastError();
-    return OA_OK;
-  }
+  // areas first, then nodes: 168 B per node; without room for them the
+  // gradients keep the ip form
+  f.edge_area = static_cast<double*>(spare_alloc((sizeof(double) * 576 + sizeof(int) * 192) * ng, m.nn));
+  if (!f.edge_area) return OA_OK;
+  f.edge_node = reinterpret_cast<int*>(f.edge_area + 576 * ng);
   k_edge_areas<<<(unsigned)((32 * ng + BLOCK - 1) / BLOCK), BLOCK, 0, f.stream>>>(m.view(), f.edge_node, f.edge_area);
   count_launches(1);
   OA_CUDA(cudaGetLastError());

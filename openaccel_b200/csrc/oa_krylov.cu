@@ -898,6 +898,27 @@ __global__ void __launch_bounds__(256) k_ell_values(int n, const int* __restrict
   for (int q = 0; q < W; ++q) out[(size_t)(i >> 5) * 32 * W + 32 * q + (i & 31)] = v[q];
 }
 
+// Bytes per row that stay free beside storage of this kind: more than a program
+// takes from the mesh on. A 24^3 flow with its solvers holds 3.2 KB per row in
+// FP64 and 2.6 in the mixed form, conduction on 17^3 nodes 3.0 and 2.5; the k
+// and omega systems add 0.5, the autotuner 0.3.
+constexpr size_t SPARE_BYTES_PER_ROW = 4096;
+
+void* spare_alloc(size_t bytes, long long rows) {
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (free_bytes < bytes || free_bytes - bytes < SPARE_BYTES_PER_ROW * (size_t)rows) return nullptr;
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+
 int ell_graph(int n, const int* h_rp, const int* rp, const int* cols, EllGraph* out, cudaStream_t st) {
   *out = EllGraph{};
   int longest = 0;
@@ -905,9 +926,8 @@ int ell_graph(int n, const int* h_rp, const int* rp, const int* cols, EllGraph* 
   const int w = longest <= 7 ? 7 : 15;
   const long long groups = (n + 31LL) / 32, slots = groups * 32 * w;
   if (longest > w || slots > 2LL * h_rp[n] + 4096) return OA_OK;
-  int* c = nullptr;
-  if (cudaMalloc(&c, sizeof(int) * (slots + groups * (w + 1)) + sizeof(uint16_t) * groups * 32) != cudaSuccess)
-    return fail(OA_ERR_CUDA, "fixed-width matrix storage: allocation failed");
+  int* c = static_cast<int*>(spare_alloc(sizeof(int) * (slots + groups * (w + 1)) + sizeof(uint16_t) * groups * 32, n));
+  if (!c) return OA_OK;
   int* delta = c + slots;
   uint16_t* mask = reinterpret_cast<uint16_t*>(delta + groups * (w + 1));
   out->w = w;

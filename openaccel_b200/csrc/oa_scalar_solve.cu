@@ -157,14 +157,11 @@ int ScalarSolve::init(const ScalarGraph& g, bool mixed) {
   if (const char* e = std::getenv("OA_IR_INNER")) inner_floor = std::atof(e);
   if (const char* e = std::getenv("OA_KRYLOV")) gcr = std::strcmp(e, "bicgstab") != 0;
   if (const char* e = std::getenv("OA_GCR_CHUNK")) gcr_chunk = std::max(2, std::atoi(e) / 2 * 2);
-  const size_t ell_bytes = (mixed ? sizeof(float) : sizeof(double)) * (size_t)std::max<long long>(1, g.ell.slots);
+  const size_t ell_bytes = (mixed ? sizeof(float) : sizeof(double)) * (size_t)g.ell.slots;
   if (n == nn && r && ell_size >= ell_bytes) return OA_OK;
   release();
   n = nn;
-  if (cudaMalloc(&ell, ell_bytes) != cudaSuccess) {
-    release();
-    return fail(OA_ERR_CUDA, "scalar solve: device allocation failed");
-  }
+  if (ell_bytes) ell = spare_alloc(ell_bytes, nn);
   ell_size = ell_bytes;
   if (cudaMalloc(&r, sizeof(double) * (nn ? nn : 1)) != cudaSuccess ||
       cudaMalloc(&r32, sizeof(float) * (nn ? nn : 1)) != cudaSuccess ||
@@ -184,13 +181,12 @@ int ScalarSolve::init(const ScalarGraph& g, bool mixed) {
 // its products and the finest level's smoothing (25 us at 2.1M rows in FP32,
 // where each of the 60 passes over the matrix saves about 10).
 int ScalarSolve::widen_matrix(const ScalarGraph& g, bool mixed, const void* A, cudaStream_t st) {
-  const bool on = g.ell.w != 0;
   k64.ell = k32.ell = g.ell;
-  k64.ell_val = on && !mixed ? ell : nullptr;
-  k32.ell_val = on && mixed ? ell : nullptr;
+  k64.ell_val = mixed ? nullptr : ell;
+  k32.ell_val = mixed ? ell : nullptr;
   amg64.set_finest(g.ell, static_cast<const double*>(k64.ell_val));
   amg32.set_finest(g.ell, static_cast<const float*>(k32.ell_val));
-  if (!on) return OA_OK;
+  if (!ell) return OA_OK;
   return mixed ? ell_values<float>(g.nn, g.rp, static_cast<const float*>(A), g.ell, static_cast<float*>(ell), st)
                : ell_values<double>(g.nn, g.rp, static_cast<const double*>(A), g.ell, static_cast<double*>(ell), st);
 }

@@ -115,12 +115,12 @@ struct ScalarSolve {
   }
 
   int init(const ScalarGraph& g, bool mixed);
-  // the solve's matrix in fixed-width storage
+  // the solve's matrix in fixed-width storage (null: none), and the bytes asked
   void* ell = nullptr;
   size_t ell_size = 0;
   int widen_matrix(const ScalarGraph& g, bool mixed, const void* A, cudaStream_t st);
   KrylovMatrix<float> matrix32(const ScalarGraph& g, const float* A) const {
-    return {g.rp, g.cols, A, g.ell, g.ell.w ? static_cast<const float*>(ell) : nullptr};
+    return {g.rp, g.cols, A, g.ell, static_cast<const float*>(ell)};
   }
   // A: const double* (mixed = false) or const float* (mixed = true); b and x
   // FP64 device vectors of g.nn; x is overwritten. refinements may be null.
