@@ -416,11 +416,10 @@ __device__ __forceinline__ void sym_face(const TF (&x)[8][3], const TF (&Uc)[8][
 // geometry (upwind advection with the same mass flows, diffusion with the
 // nodal diffusivities at the ips: phiAssemblerElemTerms.hpp:11-413, N = 1);
 // VAR 0 is the steady upwind SIMPLE assembly with nothing else in its
-// register budget. Blocks per SM, measured at 128^3: FP32 4 (1,781 us; 3: 2,192,
-// 5 spills: 1,858), FP64 3 (3,243 us in 168 registers with a few spills; 2:
-// 3,626, 4: 4,106).
-template <int LPR, bool USH, bool UGSH, class TF, int VAR = 0>
-__global__ void __launch_bounds__(BLOCK, sizeof(TF) == 4 ? (UGSH ? 4 : 3) : (UGSH ? 3 : 1))
+// register budget. Blocks per SM: FP32 4 (1,781 us at 128^3; 3: 2,192, 5 spills:
+// 1,858), FP64 2 or, with THREE, 3 (see launch_momentum).
+template <int LPR, bool USH, bool UGSH, class TF, int VAR, bool THREE>
+__global__ void __launch_bounds__(BLOCK, sizeof(TF) == 4 ? (UGSH ? 4 : 3) : (THREE ? 3 : 1))
     k_momentum(MomArgs a) {
   constexpr bool EXT = VAR == 1;
   constexpr bool TURB = VAR == 2;
@@ -1569,6 +1568,22 @@ int launch_xloc(Flow& f) {
   return OA_OK;
 }
 
+// Threads (lanes of all rows) from which the FP64 row kernel runs three blocks
+// per SM. It is bound by latency at the two blocks that its 255 registers allow;
+// in 168 registers three fit, with 1.1 KB of spills per thread. That pays where
+// tables and matrix stream from DRAM, and costs where they stay in L2 (times in
+// us, two blocks / three; 40^3 cells are 551,000 threads, 48^3 941,000):
+//   8 lanes, 40^3 cells  109 / 122, SIMPLEC 129 / 142, with k and omega 164 / 169
+//   46^3                 182 / 181          209 / 209                   257 / 247
+//   96^3               1,493 / 1,388      1,727 / 1,615               2,140 / 1,957
+//   16 lanes, 23,137 rows 74 / 80            91 / 98                    109 / 115
+//   75,025 rows          236 / 227          280 / 271                   348 / 320
+// Unshifted interpolation spills more and the line lies higher (64^3 cells, 2.2M
+// threads, 465 / 479, SIMPLEC 546 / 541; 174,273 rows of 16 lanes, 2.8M threads,
+// 548 / 544 and 653 / 626). With the high-resolution terms two blocks are the
+// faster ones throughout (40^3 148 / 175, 96^3 1,963 / 2,025).
+constexpr long long MOM_THREE_THREADS = 800000, MOM_THREE_UNSHIFTED = 2500000;
+
 int launch_momentum(Flow& f, bool mixed) {
   if (mixed) {
     if (!f.xloc32 || !f.umu32) return fail(OA_ERR_ARG, "momentum assembly: mixed-form buffers missing");
@@ -1601,21 +1616,27 @@ int launch_momentum(Flow& f, bool mixed) {
     a.urf_w_inv = 1.0 / f.urf_w;
   }
   const int var = f.turb ? 2 : (hr ? 1 : 0);
+  const bool three =
+      gs && !f.s.hr && (long long)f.mesh->nn * f.mesh->lpr >= (us ? MOM_THREE_THREADS : MOM_THREE_UNSHIFTED);
   auto go = [&](auto lanes) {
     constexpr int L = decltype(lanes)::value;
-#define OA_MOM(US, GS, T)                                                                   \
+#define OA_MOM(US, GS, T, M3)                                                               \
   if (us == US && gs == GS) {                                                               \
     if (var == 1)                                                                           \
-      k_momentum<L, US, GS, T, 1><<<g, bs, 0, f.stream>>>(a);                               \
+      k_momentum<L, US, GS, T, 1, M3><<<g, bs, 0, f.stream>>>(a);                           \
     else if (var == 2)                                                                      \
-      k_momentum<L, US, GS, T, 2><<<g, bs, 0, f.stream>>>(a);                               \
+      k_momentum<L, US, GS, T, 2, M3><<<g, bs, 0, f.stream>>>(a);                           \
     else                                                                                    \
-      k_momentum<L, US, GS, T, 0><<<g, bs, 0, f.stream>>>(a);                               \
+      k_momentum<L, US, GS, T, 0, M3><<<g, bs, 0, f.stream>>>(a);                           \
   }
     if (mixed) {
-      OA_MOM(true, true, float) OA_MOM(true, false, float) OA_MOM(false, true, float) OA_MOM(false, false, float)
+      OA_MOM(true, true, float, false) OA_MOM(true, false, float, false)
+      OA_MOM(false, true, float, false) OA_MOM(false, false, float, false)
+    } else if (three) {
+      OA_MOM(true, true, double, true) OA_MOM(false, true, double, true)
     } else {
-      OA_MOM(true, true, double) OA_MOM(true, false, double) OA_MOM(false, true, double) OA_MOM(false, false, double)
+      OA_MOM(true, true, double, false) OA_MOM(true, false, double, false)
+      OA_MOM(false, true, double, false) OA_MOM(false, false, double, false)
     }
 #undef OA_MOM
   };
