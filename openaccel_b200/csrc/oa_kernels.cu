@@ -1732,6 +1732,12 @@ static int launch_sym_grad(Flow& f, int which) {
   return OA_OK;
 }
 
+// Nodes from which the velocity gradient takes the edge form. One thread walks
+// over the three components of six edges in 6.2 us however few the nodes are;
+// the ip form with its eight lanes takes 4.1 us on 4^3 cells, 5.2 on 12^3, 6.2 on
+// 14^3 to 18^3 and 7.5 on 20^3.
+constexpr int GRADU_EDGE_NODES = 3000;
+
 int launch_gradient(Flow& f, int which) {
   const int bs = f.bs_rows;
   const int g = grid_rows(*f.mesh, bs);
@@ -1756,7 +1762,7 @@ int launch_gradient(Flow& f, int which) {
     }
   } else {
     GradArgs a{f.view(), f.U, f.gradU, f.s.grad_urf, f.edge_node, f.edge_area};
-    if (f.edge_node && f.s.u_shifted) {
+    if (f.edge_node && f.s.u_shifted && f.mesh->nn >= GRADU_EDGE_NODES) {
       k_gradient_edges<3, false><<<(f.mesh->nn + 255) / 256, 256, 0, f.stream>>>(a, nullptr, nullptr, 0.0);
     } else if (f.mesh->lpr == 16) {
       if (f.s.u_shifted) k_gradient<16, 3, true><<<g, bs, 0, f.stream>>>(a);

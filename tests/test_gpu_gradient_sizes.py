@@ -57,3 +57,10 @@ def test_velocity_correction(oracle_mod, shape, du_mode):
     gf.simple_iterate(3)
     for k in ("U", "gradP", "gradU"):
         assert rel(gf.get_field(k), oc.field(k)) < 1e-10, k
+
+
+# nodes: 2,940 and 3,000 (the velocity gradient takes the edge form from there),
+# 3,072 (whole blocks), 3,150 (78 past a block, 14 past a group), 3,328, 3,375
+@pytest.mark.parametrize("shape", [(13, 13, 14), (14, 19, 9), (15, 15, 11), (13, 14, 14), (12, 15, 15), (14, 14, 14)])
+def test_gradients_around_the_edge_forms_lowest_size(oracle_mod, shape):
+    test_gradients(oracle_mod, shape)
