@@ -89,6 +89,7 @@ void Amg<T>::release() {
   L.clear();
   if (dense_inv) cudaFree(dense_inv);
   if (dense_op) cudaFree(dense_op);
+  operator_stale = false;
   dense_inv = nullptr;
   dense_op = nullptr;
   dense_work = nullptr;
@@ -1250,6 +1251,7 @@ int Amg<T>::set_smoothing(int degree, double prolongation_damping) {
     return fail(OA_ERR_ARG, "AMG: Chebyshev degree 2..6 and prolongation damping in (0, 1.5)");
   omega_p = prolongation_damping;
   if (!smoothed) return OA_OK;
+  if (dense_op && degree != cheb_degree) operator_stale = true;
   cheb_degree = degree;
   return OA_OK;
 }

@@ -92,6 +92,12 @@ struct Amg {
   double* dense_op = nullptr;
   double* dense_work = nullptr;
   int dense_operator(cudaStream_t st);
+  bool operator_stale = false;  // formed with another Chebyshev degree than the upper levels now use
+  int refresh_operator(cudaStream_t st) {
+    if (!operator_stale) return 0;
+    operator_stale = false;
+    return dense_operator(st);
+  }
   bool ready = false;
 
   // structure from the fine graph (host arrays); device pointers of the fine
@@ -102,8 +108,9 @@ struct Amg {
   // z = M^-1 v (one V-cycle from zero initial guess); kernels return early when *done
   int apply(const T* v, T* z, const int* done, cudaStream_t st);
   // Chebyshev degree of the coarse-level smoother and prolongation damping;
-  // before set-up they shape it, after it they take effect with the next
-  // numeric phase (degree) and apply (launch count)
+  // before set-up they shape it, after it the degree takes effect with the next
+  // solve (whose caller refreshes the dense operator), the damping with the
+  // next numeric phase
   int set_smoothing(int degree, double prolongation_damping);
   // fixed-width storage of the current finest matrix (null: its CSR arrays are used)
   void set_finest(const EllGraph& g, const T* val) {

@@ -317,6 +317,11 @@ int ScalarSolve::solve(const ScalarGraph& g, bool mixed, bool amg, bool graphs, 
   if (int s = widen_matrix(g, mixed, A, st)) return s;
   if (!mixed) {
     if (int s = k64.setup(g.nn, g.rp, g.cols, g.diag, st)) return s;
+    if (amg && reuse) {
+      if (int s = amg64.refresh_operator(st)) return s;
+    } else {
+      amg64.operator_stale = false;  // the numeric phase forms it
+    }
     double* xs = nullptr;
     if (int s = k64.solve<double>(static_cast<const double*>(A), b, xs, rtol, maxit, iters, res, check_every, reuse))
       return s;
@@ -549,6 +554,7 @@ int ScalarSolve::emit(GraphBuild& gb, cudaGraph_t g, Deps& d, const ScalarGraph&
 
 int ScalarSolve::graph_prepare(cudaStream_t st) {
   if (!gs) return fail(OA_ERR_NOT_READY, "scalar solve graph: not captured");
+  if (int s = amg64.refresh_operator(st)) return s;
   gs_host->refresh_ctr = (int)solves;
   OA_CUDA(cudaMemcpyAsync(&gs->refresh_ctr, &gs_host->refresh_ctr, sizeof(int), cudaMemcpyHostToDevice, st));
   return OA_OK;
