@@ -297,7 +297,7 @@ __device__ __forceinline__ void for_rows(int n, F&& f) {
   }
 }
 
-// LPR of ELL or above: one thread per row over the fixed-width storage.
+// LPR of ELL or above (finest level): one thread per row over the fixed-width storage.
 template <class T>
 struct RowMat {
   int n;
@@ -740,7 +740,22 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1)
   }
 }
 
-// the same for kernels over a level's matrix, which may be in fixed-width storage
+// a kernel over rows, by the lanes of a row
+#define OA_LPR_LAUNCH(lpr, kernel, T, rows, st, ...)                                         \
+  do {                                                                                        \
+    if ((lpr) == 1)                                                                           \
+      kernel<T, 1><<<grid_for(rows, 1), AB, 0, st>>>(__VA_ARGS__);                            \
+    else if ((lpr) == 4)                                                                      \
+      kernel<T, 4><<<grid_for(rows, 4), AB, 0, st>>>(__VA_ARGS__);                            \
+    else if ((lpr) == 8)                                                                      \
+      kernel<T, 8><<<grid_for(rows, 8), AB, 0, st>>>(__VA_ARGS__);                            \
+    else                                                                                      \
+      kernel<T, 32><<<grid_for(rows, 32), AB, 0, st>>>(__VA_ARGS__);                          \
+    count_launches(1);                                                                        \
+  } while (0)
+
+// the same for kernels over the finest level's matrix, which may be in
+// fixed-width storage
 #define OA_MAT_LAUNCH(format, kernel, T, rows, st, ...)                                      \
   do {                                                                                        \
     const int f_ = (format);                                                                  \
@@ -757,19 +772,6 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1)
         kernel<T, ELL_STREAM + 15><<<grid_for(rows, 1), AB, 0, st>>>(__VA_ARGS__);            \
       count_launches(1);                                                                      \
     }                                                                                         \
-  } while (0)
-
-#define OA_LPR_LAUNCH(lpr, kernel, T, rows, st, ...)                                         \
-  do {                                                                                        \
-    if ((lpr) == 1)                                                                           \
-      kernel<T, 1><<<grid_for(rows, 1), AB, 0, st>>>(__VA_ARGS__);                            \
-    else if ((lpr) == 4)                                                                      \
-      kernel<T, 4><<<grid_for(rows, 4), AB, 0, st>>>(__VA_ARGS__);                            \
-    else if ((lpr) == 8)                                                                      \
-      kernel<T, 8><<<grid_for(rows, 8), AB, 0, st>>>(__VA_ARGS__);                            \
-    else                                                                                      \
-      kernel<T, 32><<<grid_for(rows, 32), AB, 0, st>>>(__VA_ARGS__);                          \
-    count_launches(1);                                                                        \
   } while (0)
 
 // ---------------------------------------------------------------------------
@@ -1190,13 +1192,13 @@ int Amg<T>::apply(const T* v, T* z, const int* done, cudaStream_t st) {
     const T* b = l == 0 ? v : lv.b;
     const RowMat<T> m = level_matrix(lv);
     if (lv.cheb) {
-      OA_MAT_LAUNCH(level_format(lv), k_cheb_first, T, lv.n, st, m, lv.dinv, b, lv.coef, lv.cr, lv.cd1, lv.t, done);
+      OA_LPR_LAUNCH(lv.lpr_a, k_cheb_first, T, lv.n, st, m, lv.dinv, b, lv.coef, lv.cr, lv.cd1, lv.t, done);
       for (int k = 2; k < cheb_degree; ++k) {
         const T* din = (k & 1) ? lv.cd0 : lv.cd1;
         T* dout = (k & 1) ? lv.cd1 : lv.cd0;
-        OA_MAT_LAUNCH(level_format(lv), k_cheb_next, T, lv.n, st, m, lv.dinv, din, lv.coef, k, lv.cr, dout, lv.t, done);
+        OA_LPR_LAUNCH(lv.lpr_a, k_cheb_next, T, lv.n, st, m, lv.dinv, din, lv.coef, k, lv.cr, dout, lv.t, done);
       }
-      OA_MAT_LAUNCH(level_format(lv), k_resid, T, lv.n, st, m, b, lv.t, lv.r, done);
+      OA_LPR_LAUNCH(lv.lpr_a, k_resid, T, lv.n, st, m, b, lv.t, lv.r, done);
     } else {
       OA_MAT_LAUNCH(level_format(lv), k_smooth_resid, T, lv.n, st, m, lv.dinv, b, lv.t, lv.r, omega, done);
     }
@@ -1231,11 +1233,11 @@ int Amg<T>::apply(const T* v, T* z, const int* done, cudaStream_t st) {
     const RowMat<T> p = {lv.n, lv.p_rp, lv.p_cols, lv.pv, nullptr, nullptr};
     OA_LPR_LAUNCH(lv.lpr_p, k_prolong_add, T, lv.n, st, p, xc, lv.t, alpha, done);
     if (lv.cheb) {
-      OA_MAT_LAUNCH(level_format(lv), k_cheb_start, T, lv.n, st, m, lv.dinv, b, lv.t, lv.coef, lv.cr, lv.cd0, x, done);
+      OA_LPR_LAUNCH(lv.lpr_a, k_cheb_start, T, lv.n, st, m, lv.dinv, b, lv.t, lv.coef, lv.cr, lv.cd0, x, done);
       for (int k = 1; k < cheb_degree; ++k) {
         const T* din = (k & 1) ? lv.cd0 : lv.cd1;
         T* dout = (k & 1) ? lv.cd1 : lv.cd0;
-        OA_MAT_LAUNCH(level_format(lv), k_cheb_next, T, lv.n, st, m, lv.dinv, din, lv.coef, k, lv.cr, dout, x, done);
+        OA_LPR_LAUNCH(lv.lpr_a, k_cheb_next, T, lv.n, st, m, lv.dinv, din, lv.coef, k, lv.cr, dout, x, done);
       }
     } else {
       OA_MAT_LAUNCH(level_format(lv), k_post_smooth, T, lv.n, st, m, lv.dinv, b, lv.t, x, omega, done);

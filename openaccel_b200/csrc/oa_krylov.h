@@ -11,7 +11,7 @@ namespace oa {
 // Device scalars of one Krylov solve (read by every iteration kernel).
 struct KScal {
   double rho, alpha, omega, bnorm, rnorm;
-  double d0, d1, d2;  // reduced dots of the current phase
+  double d0;  // rh.r of the current BiCGStab iteration
   double rtol;
   int maxit;
   int done, iters, status;
