@@ -22,6 +22,7 @@ from openaccel_b200 import meshgen
 from openaccel_b200 import runtime as rt
 
 from .test_amg_symbolic import _lists, harness  # noqa: F401
+from .test_gpu_node_orders import renumber
 
 COARSEST, CHEB_ROWS = 256, 50000
 
@@ -159,6 +160,26 @@ PRECISIONS = pytest.mark.parametrize("prec", [rt.OA_PREC_FP64, rt.OA_PREC_MIXED]
 def test_hex_blocks(harness, shape, rows, prec):  # noqa: F811
     f, A, b, solved = pressure(meshgen.cavity(shape, perturb=0.2), prec)
     assert not csr_refused(check(harness, f, A, b, solved, prec, rows))
+
+
+# 256 rows, one more than a multiple of 32 (225) and of 256 (513)
+@pytest.mark.gpu
+@PRECISIONS
+@pytest.mark.parametrize("shape", [(7, 7, 3), (4, 4, 8), (2, 8, 18)])
+def test_group_and_block_edges(harness, shape, prec):  # noqa: F811
+    f, A, b, solved = pressure(meshgen.cavity(shape), prec)
+    assert not csr_refused(check(harness, f, A, b, solved, prec))
+
+
+# columns instead of distances in all or some groups; the large ones with
+# streaming loads in FP64
+@pytest.mark.gpu
+@PRECISIONS
+@pytest.mark.parametrize("order", ["half", "random"])
+@pytest.mark.parametrize("shape", [(20, 20, 20), (85, 85, 85)])
+def test_node_orders(harness, shape, order, prec):  # noqa: F811
+    f, A, b, solved = pressure(renumber(meshgen.cavity(shape, perturb=0.2), order), prec)
+    assert not csr_refused(check(harness, f, A, b, solved, prec))
 
 
 @pytest.mark.gpu
