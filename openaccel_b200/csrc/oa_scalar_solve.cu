@@ -243,6 +243,9 @@ void ScalarSolve::release_segments() {
   seg_out = Segments{};
   k64.seg = Segments{};
   k32.seg = Segments{};
+  // captured chunks hold the segments' addresses, or no segment tests at all
+  k64.drop_graph();
+  k32.drop_graph();
 }
 
 void ScalarSolve::release() {

@@ -2,7 +2,8 @@
 // without a GPU (LD_PRELOAD). Device memory is host memory of a settable
 // amount, beyond which cudaMalloc returns cudaErrorMemoryAllocation; kernels do
 // nothing. tests/test_memory_limit.py runs the library's host side on it to see
-// which calls still succeed when device memory is short.
+// which calls still succeed when device memory is short, tests/test_host_state.py
+// what the host side captures and launches.
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -12,6 +13,8 @@
 static std::map<void*, size_t> g_blocks;
 static size_t g_used = 0, g_peak = 0, g_limit = ~size_t(0) / 2;
 static thread_local cudaError_t g_last = cudaSuccess;
+static int g_captures = 0;       // stream captures begun
+static unsigned g_cluster = 16;  // largest cluster that can be placed
 
 static cudaError_t set(cudaError_t e) {
   if (e != cudaSuccess) g_last = e;
@@ -20,6 +23,8 @@ static cudaError_t set(cudaError_t e) {
 
 extern "C" {
 void fake_limit(size_t bytes) { g_limit = bytes; }
+void fake_max_cluster(unsigned n) { g_cluster = n; }
+int fake_captures() { return g_captures; }
 size_t fake_used() { return g_used; }
 size_t fake_peak() {
   const size_t p = g_peak;
@@ -61,7 +66,27 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
 cudaError_t cudaMemset(void* d, int v, size_t n) { return std::memset(d, v, n), cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return std::memset(d, v, n), cudaSuccess; }
 cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) { return cudaSuccess; }
+static bool placeable(const cudaLaunchConfig_t* c) {
+  for (unsigned k = 0; k < c->numAttrs; ++k)
+    if (c->attrs[k].id == cudaLaunchAttributeClusterDimension && c->attrs[k].val.clusterDim.x > g_cluster) return false;
+  return true;
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*, void**) {
+  return placeable(c) ? cudaSuccess : set(cudaErrorInvalidClusterSize);
+}
+cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t* c) {
+  return *n = placeable(c) ? 1 : 0, cudaSuccess;
+}
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return ++g_captures, cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
+  return *g = reinterpret_cast<cudaGraph_t>(16), cudaSuccess;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+  return *e = reinterpret_cast<cudaGraphExec_t>(16), cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
   return *s = reinterpret_cast<cudaStream_t>(16), cudaSuccess;

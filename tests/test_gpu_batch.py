@@ -98,3 +98,21 @@ def test_batch_graph_iterations_match_eager():
     np.testing.assert_array_equal(u1, u2)
     np.testing.assert_array_equal(p1, p2)
     assert [s["pc_iters"] for s in s1] == [s["pc_iters"] for s in s2]
+
+
+@pytest.mark.parametrize("prec", [rt.OA_PREC_FP64, rt.OA_PREC_MIXED])
+def test_reference_nodes_set_again_between_solves(prec):
+    # captured solver chunks belong to one set of segments
+    b = meshgen.batch_cavities(sizes=[4, 6, 5], seed=7)
+    runs = []
+    for again in (0, 2):
+        gm, gf = _gpu_flow(b.mesh, b.mu, b.ref_nodes, precision=prec, use_graphs=1)
+        gf.assemble_pcorr()
+        out = []
+        for _ in range(3):
+            out.append(gf.solve("pcorr", 1e-10, 500)[0])
+            for _ in range(again):
+                gf.set_reference_nodes(b.ref_nodes)
+        runs.append(out)
+    for x, y in zip(*runs):
+        np.testing.assert_array_equal(x, y)
