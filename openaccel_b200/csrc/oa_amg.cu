@@ -560,22 +560,41 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Launch of a kernel as one cluster of CLUSTER_BLOCKS blocks (more than the
-// portable 8: Amg::set-up opts the kernels in on its device).
+// A launch as one cluster of CLUSTER_BLOCKS blocks, more than the portable 8.
+struct ClusterLaunch {
+  cudaLaunchConfig_t c = {};
+  cudaLaunchAttribute at[1];
+  explicit ClusterLaunch(cudaStream_t st) {
+    c.gridDim = CLUSTER_BLOCKS;
+    c.blockDim = CLUSTER_THREADS;
+    c.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CLUSTER_BLOCKS;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+  }
+};
+
+// Opts a kernel in on the current device; false where such a cluster cannot be
+// placed there (a slice of a GPU).
+template <class K>
+static bool cluster_fits(K kernel) {
+  const ClusterLaunch l(nullptr);
+  int n = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &l.c) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return n > 0;
+}
+
 template <class K, class... A>
 static int launch_cluster(K kernel, cudaStream_t st, const A&... args) {
-  cudaLaunchConfig_t c = {};
-  c.gridDim = CLUSTER_BLOCKS;
-  c.blockDim = CLUSTER_THREADS;
-  c.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CLUSTER_BLOCKS;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  c.attrs = at;
-  c.numAttrs = 1;
-  OA_CUDA(cudaLaunchKernelEx(&c, kernel, args...));
+  const ClusterLaunch l(st);
+  OA_CUDA(cudaLaunchKernelEx(&l.c, kernel, args...));
   count_launches(1);
   return OA_OK;
 }
@@ -927,7 +946,7 @@ int Amg<T>::setup(int n, const int* h_rp, const int* h_cols, const int* h_diag, 
   coarse_n = L.back().n;
   if (cudaMalloc(&dense_inv, sizeof(double) * 2 * (size_t)coarse_n * coarse_n) != cudaSuccess)
     return fail(OA_ERR_CUDA, "AMG: dense coarse allocation failed");
-  OA_CUDA(cudaFuncSetAttribute(k_power_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  power_cluster = cluster_fits(k_power_cluster<T>);
   // the dense operator's level and the workspace its columns are formed in
   tail = (int)L.size() - 1;
   // (the finest matrix is always the current one, and an FP32 cycle rounds its
@@ -956,7 +975,7 @@ int Amg<T>::numeric(const T* A_fine, cudaStream_t st) {
     AmgLevel<T>& v = L[l];
     k_dinv<T><<<(v.n + AB - 1) / AB, AB, 0, st>>>(v.n, v.rp, v.diag, v.A, v.dinv);
     count_launches(1);
-    if (v.cheb && (size_t)v.nnz * (sizeof(T) + sizeof(int)) <= POWER_CLUSTER_BYTES) {
+    if (v.cheb && power_cluster && (size_t)v.nnz * (sizeof(T) + sizeof(int)) <= POWER_CLUSTER_BYTES) {
       if (int s = launch_cluster(k_power_cluster<T>, st, level_matrix(v), v.nnz, (const T*)v.dinv, v.est, v.pw_v, v.pw_w,
                                  v.pw_part, cheb_ratio, v.coef))
         return s;

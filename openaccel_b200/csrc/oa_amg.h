@@ -85,6 +85,7 @@ struct Amg {
   int cheb_degree = 3;
   int cheb_rows = 50000;
   double cheb_ratio = 30.0;
+  bool power_cluster = false;  // small levels' power iteration in one cluster of 16 blocks
   // the cycle from level `tail` down is one dense operator [n][n] (row-major),
   // formed by the numeric phase in dense_work (both in one allocation); null
   // where tail is the coarsest level, whose operator is its inverse itself

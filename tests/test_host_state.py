@@ -35,3 +35,15 @@ for nodes in (None, b.ref_nodes, None, b.ref_nodes):
     captures.append(fake.fake_captures())
 assert captures == [1, 2, 2, 3], captures
 """)
+
+
+def test_solve_without_room_for_a_large_cluster(fake):  # noqa: F811
+    """The power iteration of small levels takes a cluster of more than the
+    portable 8 blocks only where one can be placed."""
+    run(fake, r"""
+fake.fake_max_cluster(8)
+f = rt.Flow(rt.Mesh(meshgen.cavity(12)), rt.default_settings())
+f.initialize()
+f.assemble_pcorr()
+f.solve("pcorr", 1e-8, 4)
+""")
