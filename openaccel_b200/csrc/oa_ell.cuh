@@ -6,8 +6,10 @@
 // row pointer in its chain of dependent loads, and has all W slots in flight at
 // once. W is a compile-time constant, for the two row lengths of the stencils
 // this library assembles: 7 (a node of a hex block and its edge neighbours) and
-// 15 (a node of a block split into Kuhn tets). Other graphs keep CSR, and so
-// does one that the padding would more than double.
+// 15 (a node of a block split into Kuhn tets, or of hex blocks around an axis). A
+// graph takes 7 where no row is longer, 15 where none is longer than that, and
+// keeps CSR otherwise, where the slots are more than 2 nnz + 4096 and where device
+// memory is short.
 //
 // In a block's numbering the 32 rows of a group have their columns at the same
 // few distances, so a group keeps the distances once where W of them hold all its
@@ -19,7 +21,8 @@
 // 129^3 rows FP32 32.8 and 20.7; a run-time width lost most of it (20.7 and 28.9
 // us). On 129^3 rows FP32 with columns and with distances: smoothing step with
 // residual 24.7 and 22.8 us, smoothing step 23.8 and 20.9, product in GCR 26.6
-// and 24.7. Absent slots have value 0 and a column of the row itself.
+// and 24.7. Absent slots have value 0 and a column that the row reads anyway: the
+// row itself by distances, the row's first one by columns.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -1187,7 +1187,7 @@ __global__ void __launch_bounds__(BLOCK) k_gradient(GradArgs a) {
 
 // The same with shifted interpolation on a block mesh. The value at an ip is
 // then the mean of its edge's two nodes and walls add nothing, so the ips of
-// an edge share it and their area vectors sum once per mesh: one thread per
+// an edge share it and their area vectors sum once per flow: one thread per
 // node reads six edges instead of eight lanes reading 24 ips. The ip form was
 // bound by L1 (91 % of its wavefronts: strided area loads); this one streams
 // 168 B of edges per node. A warp's gradients pass through shared memory so

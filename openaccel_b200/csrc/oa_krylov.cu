@@ -6,9 +6,10 @@
 // The reference hands its systems to liblinsolve (PETSc / Trilinos / HYPRE,
 // src/equation/linearSystem.h:416-462), which is absent from the reference
 // checkout; the algorithm here is the published one. All scalars live on the
-// device and every reduction is a fixed two-stage tree (block partials, then
-// an ordered single-block sum), so results are bitwise reproducible run to
-// run. A device "done" flag lets chunks of iterations be launched without
+// device and every reduction is a fixed two-stage tree (block partials, which
+// every block of the kernel that needs the sum adds in one order; segments of a
+// batch close in the last block, in chunk order), so results are bitwise
+// reproducible run to run. A device "done" flag lets chunks of iterations be launched without
 // host round trips; kernels after convergence return immediately.
 #include <cuda_runtime.h>
 
@@ -46,8 +47,11 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // Fixed-order two-stage reductions: a partial per block, and every block of
 // the kernel that needs the sum adds the partials in the same order. On a
-// 16^3 cavity this costs 0.1 to 0.2 us per kernel; a ticket with the last block
-// adding up cost 1.6 us, a kernel of one block for the sum 3 to 4.
+// 16^3 cavity (20 partials) this costs 0.1 to 0.2 us per kernel; a ticket with the
+// last block adding up cost 1.6 us, a kernel of one block for the sum 3 to 4. With
+// all 2,048 partials it costs what it replaces: on 129^3 rows in FP32 k_gcr_orth,
+// k_gcr_update and k_end_iter take 18.9, 23.9 and 4.4 us, with kernels of one
+// block between them they took 18.1, 16.5 and 3 x 4.3.
 template <int NV>
 __device__ __forceinline__ void block_partials(double (&v)[NV], double* partials) {
   __shared__ double sh[NV][KB / 32];
@@ -293,7 +297,10 @@ __device__ __forceinline__ double scalar_row(const ScalarMat<TM>& m, int i, cons
     default: call(1);                  \
   }
 
-// y = A x for a BSR matrix with BxB row-major blocks.
+// y = A x for a BSR matrix with BxB row-major blocks. The scalar row products run
+// 8 blocks per SM (32 registers): a pass of the mixed 128^3 cavity takes 39.1 ms,
+// with 6 blocks 39.7. In FP64 width 7 spills 68 to 80 B per thread at 8, and 6 is
+// the faster one (16^3 3.78 against 3.69 ms, 96^3 22.7 against 21.8).
 // STEP 1: partial w.y with w = rh; STEP 2: partials y.w and y.y with w = s.
 template <int B, class TM, class TV, int STEP, int FORMAT>
 __global__ void __launch_bounds__(KB, B == 1 ? 8 : 1) k_spmv(int nn, ScalarMat<TM> M, const TV* __restrict__ x, TV* __restrict__ y,
